@@ -8,6 +8,7 @@
 
 #include "../../include/rkf_cuda_testing.h"
 #include "ctx.h"
+#include "settle.h"
 #include "edit.h"
 #include "empty_dist.h"
 
@@ -88,8 +89,22 @@ ObjDev make_objdev(const rkf_gpu_object& o, uint32_t top_off, uint32_t has_flat)
   for (int a = 0; a < 4; ++a) d.params[a] = o.sdf_params[a];
   for (int a = 0; a < 3; ++a) {
     d.tv[a] = static_cast<int>(o.brick_map_dims[a]) * 8;
+    d.last[a] = static_cast<float>(d.tv[a] - 1);
     d.bdims[a] = o.brick_map_dims[a];
     d.tdim[a] = (o.brick_map_dims[a] + 7) / 8;
+  }
+  d.mirror = 63;
+  while (d.mirror < (1 << 20) && (d.mirror < d.tv[0] - 1 || d.mirror < d.tv[1] - 1 || d.mirror < d.tv[2] - 1))
+    d.mirror = 2 * d.mirror + 1;
+  for (int a = 0; a < 3; ++a) {
+    // (the geometry box is object-local; the walk's margin covers the roundings)
+    d.core_lo[a] = 0.0f;
+    d.core_hi[a] = d.last[a];
+    if (d.has_geom && d.vs > 0.0f) {
+      d.core_lo[a] = std::fmax(d.core_lo[a], (d.gmin[a] + d.half_gs[a]) / d.vs - 0.5f);
+      d.core_hi[a] = std::fmin(d.core_hi[a], (d.gmax[a] + d.half_gs[a]) / d.vs - 0.5f);
+    }
+    d.mag[a] = std::fabs(d.m[12 + a]) + d.gs[a];
   }
   d.top_off = top_off;
   d.map_off = o.brick_map_offset;
@@ -122,6 +137,7 @@ SceneDev Ctx::scene_dev() const {
   s.top = top.as<uint32_t>();
   s.empty_dist = empty_dist.as<uint8_t>();
   s.leaves = leaves.as<uint32_t>();
+  s.leaf_dist = leaf_dist.as<uint8_t>();
   s.flat_maps = flat_maps.as<uint32_t>();
   s.objs = objdev.as<ObjDev>();
   s.n_objs = obj_count();
@@ -203,15 +219,21 @@ rkf_status Ctx::ensure_leaf_capacity(uint32_t need) {
   if (leaves_frozen) return fail(RKF_OOM, "index leaf capacity reserved for the serving session is exhausted");
   uint32_t cap = leaf_cap ? leaf_cap : 64;
   while (cap < need) cap *= 2;
-  DevBuf nb;
+  DevBuf nb, nd;
   rkf_status st = nb.alloc(static_cast<size_t>(cap) * 512 * 4);
+  if (st == RKF_OK) st = nd.alloc(static_cast<size_t>(cap) * 512);
   if (st != RKF_OK) return st;
-  if (n_leaves)
+  if (n_leaves) {
     RKF_CUDA_TRY(cudaMemcpyAsync(nb.p, leaves.p, static_cast<size_t>(n_leaves) * 2048,
                                  cudaMemcpyDeviceToDevice, stream));
+    RKF_CUDA_TRY(cudaMemcpyAsync(nd.p, leaf_dist.p, static_cast<size_t>(n_leaves) * 512,
+                                 cudaMemcpyDeviceToDevice, stream));
+  }
   RKF_CUDA_TRY(cudaStreamSynchronize(stream));
   std::swap(leaves.p, nb.p);
   std::swap(leaves.bytes, nb.bytes);
+  std::swap(leaf_dist.p, nd.p);
+  std::swap(leaf_dist.bytes, nd.bytes);
   leaf_cap = cap;
   return RKF_OK;
 }
@@ -416,6 +438,9 @@ rkf_status rkf_create(const rkf_config* cfg, rkf_ctx** out) {
     cudaStreamDestroy(c->stream);
     return st;
   }
+  // room for the settling passes of a 1920x1080 view, so that a first view does
+  // not wait for it; larger ones grow it, and without it views march alone
+  if (c->settle_buf.alloc(settle_bytes(1920u * 1080u, 32)) != RKF_OK) cudaGetLastError();
   c->free_slots.resize(cap);
   for (size_t i = 0; i < cap; ++i) c->free_slots[i] = static_cast<uint32_t>(cap - 1 - i);
   c->tuning = rkf_batch_tuning{4, 8, 32, 64, 0, 256, 32, 0, 0};
@@ -613,17 +638,27 @@ rkf_status rkf_objects_import(rkf_ctx* ctx, const rkf_gpu_object* objects, uint3
   const uint32_t nl = static_cast<uint32_t>(leaf_host.size() / 512);
   uint32_t cap = 64;
   while (cap < nl) cap *= 2;
-  DevBuf nleaves, ntop, nfield;
+  DevBuf nleaves, nleafd, ntop, nfield;
   rkf_status st = nleaves.alloc(static_cast<size_t>(cap) * 2048);
+  if (st == RKF_OK) st = nleafd.alloc(static_cast<size_t>(cap) * 512);
   if (st == RKF_OK) st = ntop.alloc(std::max<size_t>(top.size(), 1) * 4);
   if (st == RKF_OK) st = nfield.alloc(std::max<size_t>(top.size(), 1));
   if (st != RKF_OK) return st;
   if (nl)
     RKF_CUDA_TRY(cudaMemcpy(nleaves.p, leaf_host.data(), leaf_host.size() * 4, cudaMemcpyHostToDevice));
   if (!top.empty()) RKF_CUDA_TRY(cudaMemcpy(ntop.p, top.data(), top.size() * 4, cudaMemcpyHostToDevice));
-  for (const ObjDev& d : od)
+  for (const ObjDev& d : od) {
     if ((st = build_empty_dist(d, ntop.as<uint32_t>(), nfield.as<uint8_t>(), c->stream)) != RKF_OK) return st;
     c->counted(3);
+    if (d.sdf_type != RKF_SDF_VOXELIZED) continue;
+    std::vector<uint32_t> blocks;  // the object's leaf blocks
+    for (uint32_t b = d.top_off; b < d.top_off + d.tdim[0] * d.tdim[1] * d.tdim[2]; ++b)
+      if (top[b] < RKF_INTERIOR_SLOT) blocks.push_back(b);
+    if ((st = build_leaf_dist(d, ntop.as<uint32_t>(), nleaves.as<uint32_t>(), nleafd.as<uint8_t>(), blocks,
+                              c->stream)) != RKF_OK)
+      return st;
+    c->counted(blocks.empty() ? 0 : 1);
+  }
   std::vector<rkf_gpu_object> objects0(objects, objects + n);
   std::swap(c->objects, objects0);
   std::swap(c->objdev_host, od);
@@ -634,6 +669,8 @@ rkf_status rkf_objects_import(rkf_ctx* ctx, const rkf_gpu_object* objects, uint3
   }
   std::swap(c->leaves.p, nleaves.p);
   std::swap(c->leaves.bytes, nleaves.bytes);
+  std::swap(c->leaf_dist.p, nleafd.p);
+  std::swap(c->leaf_dist.bytes, nleafd.bytes);
   c->leaf_cap = cap;
   c->n_leaves = nl;
   c->free_leaves.clear();
@@ -702,7 +739,7 @@ rkf_status rkf_scene_info_get(rkf_ctx* ctx, rkf_scene_info* out) {
   out->pool_capacity = c->capacity;
   out->leaf_blocks = c->n_leaves;
   out->device_bytes = c->dist_f16.bytes + c->dist_f32.bytes + c->dist_u8.bytes + c->brick_step.bytes +
-                      c->mat.bytes + c->blend.bytes + c->aos.bytes + c->top.bytes + c->empty_dist.bytes + c->leaves.bytes +
+                      c->mat.bytes + c->blend.bytes + c->aos.bytes + c->top.bytes + c->empty_dist.bytes + c->leaves.bytes + c->leaf_dist.bytes +
                       c->flat_maps.bytes + c->objdev.bytes;
   out->epoch = c->epoch;
   return RKF_OK;

@@ -90,6 +90,7 @@ struct Ctx {
   uint64_t top_len = 0;
   DevBuf empty_dist;  // u8 per top cell: empty-space distance field (empty_dist.h)
   DevBuf leaves;
+  DevBuf leaf_dist;  // u8 per leaf entry: empty-space distance at brick resolution (empty_dist.h)
   uint32_t n_leaves = 0, leaf_cap = 0;
   std::vector<uint32_t> free_leaves;  // leaf numbers below n_leaves that no epoch references
   bool leaves_frozen = false;  // set while serving: the leaf buffer must not move
@@ -132,6 +133,7 @@ struct Ctx {
   cudaEvent_t band_ev[kMaxBands] = {};
   cudaEvent_t segs_ev = nullptr;
   DevBuf order_buf;  // heaviest-first tile order of views (tile_order.h)
+  DevBuf settle_buf; // lists of the settling passes (settle.h)
   DevBuf counters;   // work counters of the persistent kernels
   DevBuf seg_buf;    // segment table of the persistent kernel
 

@@ -54,6 +54,12 @@ struct ObjDev {
   uint32_t div_ok;      // 1: exact_div_vs == IEEE x/vs verified on [lo, max(hi)]
   uint32_t translate_only;  // inverse_world is identity in its linear part
   float vs2;            // vs * 2 (INTERIOR value of the stepping sampler)
+  float last[3];        // tv - 1
+  // the walk through EMPTY boxes, in voxel-centre coordinates: 2^n - 1 >= every
+  // voxel index (at least 63; index v mirrors to v ^ mirror), the grid's border
+  // voxels clipped to the geometry box, and |translation| + grid size (metres)
+  int mirror;
+  float core_lo[3], core_hi[3], mag[3];
 };
 
 // x / vs rounded to nearest even, by one Markstein correction step of the
@@ -67,6 +73,23 @@ __device__ __forceinline__ float exact_div_vs(float x, float vs, float rcp) {
   return __fmaf_rn(e, rcp, q0);
 }
 
+// floor(v) and v - floor(v), for |v| < 2^22: adding 1.5 * 2^23 rounds v to the
+// nearest integer, whose difference from v is exact, and a negative difference
+// is one integer too high.  The same bits as floorf, v - floorf(v) and the
+// conversion (the sign of a zero difference aside, which no mix sees), in
+// full-rate instructions; floorf and the conversion issue at a quarter rate.
+constexpr float kIntMagic = 12582912.0f;
+__device__ __forceinline__ float up_frac(float d) { return d < 0.0f ? __fadd_rn(d, 1.0f) : d; }
+__device__ __forceinline__ float floor_frac(float v, int& i) {
+  const float m = __fadd_rn(v, kIntMagic);
+  const float d = __fsub_rn(v, __fsub_rn(m, kIntMagic));
+  i = __float_as_int(m) - 0x4B400000 - (d < 0.0f ? 1 : 0);
+  return up_frac(d);
+}
+__device__ __forceinline__ float frac_of(float v) {
+  return up_frac(__fsub_rn(v, __fsub_rn(__fadd_rn(v, kIntMagic), kIntMagic)));
+}
+
 struct SceneDev {
   const uint16_t* __restrict__ dist_f16;
   const float* __restrict__ dist_f32;
@@ -78,6 +101,7 @@ struct SceneDev {
   const uint32_t* __restrict__ top;
   const uint8_t* __restrict__ empty_dist;  // per top cell, see empty_dist.h
   const uint32_t* __restrict__ leaves;
+  const uint8_t* leaf_dist;  // per leaf entry, see empty_dist.h (edits lower it while older epochs read it)
   const uint32_t* __restrict__ flat_maps;
   const ObjDev* __restrict__ objs;
   uint32_t n_objs;
@@ -164,6 +188,19 @@ __device__ __forceinline__ uint32_t lookup2(const SceneDev& s, const ObjDev& o, 
   const uint32_t t = __ldg(s.top + top_index(o, bx, by, bz));
   if (t >= RKF_INTERIOR_SLOT) return t;
   return __ldg(s.leaves + static_cast<size_t>(t) * 512 + (bx & 7) + (by & 7) * 8 + (bz & 7) * 64);
+}
+
+// The empty-space distance at brick resolution (empty_dist.h).  An edit lowers
+// the bytes of blocks it did not copy while marches of older epochs read them
+// (any value they see is valid for them): relaxed accesses, which the memory
+// model allows to run side by side.
+__device__ __forceinline__ uint32_t load_leaf_dist(const uint8_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_leaf_dist(uint8_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u8 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // ---------------------------------------------------------------------------

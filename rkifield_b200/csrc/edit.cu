@@ -447,11 +447,13 @@ rkf_status apply_edit(Ctx* c, const rkf_edit_op& op, cudaStream_t st, EditOutcom
     }
   }
   if ((s2 = c->ensure_leaf_capacity(c->n_leaves + appended)) != RKF_OK) return s2;
+  const std::vector<uint32_t> around = blocks_around(od, blocks);  // their brick distances change too
   Temp g;
-  if ((s2 = g.get(scratch, static_cast<size_t>(nb) * (4 + 4 + 2048) + 256)) != RKF_OK) return s2;
+  if ((s2 = g.get(scratch, static_cast<size_t>(nb) * (4 + 4 + 2048) + around.size() * 4 + 256)) != RKF_OK) return s2;
   uint32_t* d_blocks = g.as<uint32_t>();
   uint32_t* d_topv = d_blocks + nb;
   uint32_t* d_leafs = d_topv + nb;
+  uint32_t* d_around = d_leafs + static_cast<size_t>(nb) * 512;
   RKF_CUDA_TRY(cudaMemcpyAsync(d_blocks, blocks.data(), nb * 4ull, cudaMemcpyHostToDevice, st));
   detail::k_gather_blocks<<<nb, 128, 0, st>>>(c->top.as<uint32_t>(), c->leaves.as<uint32_t>(), d_blocks, nb,
                                               d_topv, d_leafs);
@@ -491,7 +493,12 @@ rkf_status apply_edit(Ctx* c, const rkf_edit_op& op, cudaStream_t st, EditOutcom
   uint8_t* nfield = into ? out->field_dst : out->new_empty_dist.as<uint8_t>();
   RKF_CUDA_TRY(cudaMemcpyAsync(nfield, c->empty_dist.p, c->top_len, cudaMemcpyDeviceToDevice, st));
   if ((s2 = lower_empty_dist(od, nfield, d_blocks, blocks, st)) != RKF_OK) return s2;
-  c->counted(1);
+  // and the brick distances of the new leaves and of the leaves next to them
+  RKF_CUDA_TRY(cudaMemcpyAsync(d_around, around.data(), around.size() * 4, cudaMemcpyHostToDevice, st));
+  if ((s2 = enqueue_leaf_dist(od, ntop, c->leaves.as<uint32_t>(), c->leaf_dist.as<uint8_t>(), d_around,
+                              static_cast<uint32_t>(around.size()), st)) != RKF_OK)
+    return s2;
+  c->counted(2);
   c->n_leaves += appended;
   // the reference flat map (read only by the plain march) is updated in place
   if (od.has_flat && !c->flat_host.empty()) {

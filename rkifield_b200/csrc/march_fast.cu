@@ -30,6 +30,8 @@
 #include "march.h"
 #include "f32x2.cuh"
 #include "sampler.cuh"
+#include "walk.cuh"
+#include "settle.h"
 #include "tiled.h"
 #include "tile_order.h"
 
@@ -37,9 +39,10 @@ namespace rkf {
 
 namespace detail {
 
-enum : uint32_t { ST_IDLE = 0, ST_MARCH, ST_BISECT, ST_NORMAL, ST_EPI, ST_SHADOW };
-
-constexpr uint32_t kFull = 0xFFFFFFFFu;
+// What a lane's ray is doing: nothing, marching (towards a surface, or a
+// light), bisecting an overstep, taking the samples of a hit's normal, or done
+// with its outputs still to write.
+enum : uint32_t { ST_IDLE = 0, ST_MARCH, ST_SHADOW, ST_BISECT, ST_NORMAL, ST_EPI };
 
 // Per-lane ray state that is read or written only when a ray starts, hits
 // or ends.
@@ -47,86 +50,18 @@ struct ColdState {
   uint32_t seg, idx, hit_obj, sub;
   float lo, hi, mat_t, gpos, shadow;
   uint32_t tile_base, tile_count;  // tiled strategy: the ray's object list (kNoTiles: every object)
+  float g[3];                // the normal's central differences
+  float sdf_hit;             // the hit's own sample (motion plane)
   bool hit, bisected, mat_ok;
   // multi-object empty-space path: bits 0-7, the voxelized objects of the
   // path (KParams::ev) whose EMPTY runs the ray may take (under the tiled
   // strategy, those its object list holds); bits 8-15, the one whose cube
-  // the ray is in (its last successful probe).  (Also makes an odd number of
-  // words per lane: a warp's accesses hit 32 distinct banks.)
+  // the ray is in (its last successful probe).  Single-object variants: how
+  // the ray ends if its walk reaches its target (1 past tmax, 2 out of steps).
+  // (An odd number of words per lane: a warp's accesses hit 32 distinct banks.)
   uint32_t vox_listed;
 };
 static_assert(sizeof(ColdState) % 8 == 4, "ColdState must span an odd number of 32-bit words");
-
-// Multi-object empty-space path.  Each analytic primitive lies inside a ball
-// of radius R around its local origin (sphere r, box |b|, capsule |r|+|h|,
-// torus |R|+|r|, cylinder |(r, h)|), and its exact distance is at least |l|-R
-// at a local position l.  With c the local origin in world space, sigma a
-// lower bound of the smallest singular value of inverse_world's linear part
-// and s the object's min_scale, the FP32 value of evaluate_object at a world
-// position p is at least (sigma*|p - c| - R - rounding)*s.  The host folds
-// the voxelized object's largest EMPTY value and bounds of every rounding
-// (the object's own evaluation, the ray's position, this centre's rounding)
-// into a radius a + b*P, P = |o| + |d|*|tmax| bounding the magnitude of a
-// ray's positions: outside that ball the object's value exceeds every EMPTY
-// value, so wherever the voxelized object samples EMPTY, the minimum over
-// the scene is that sample, bit for bit.
-struct FarBall {
-  float c[3];     // world-space centre (half-space: the coefficients G)
-  float a, b;     // radius a + b * P (box: margin a + b * P beyond the half extents;
-                  // half-space: G.w + H <= a + b * P)
-  uint32_t path;  // the object's index in the empty-space path (KParams::ev), or ~0u
-  float h[3];     // box: world-space half extents (half-space: h[0] = H)
-  uint32_t box;   // 1: an axis-aligned box around c instead of a ball; 2: a half-space
-};
-
-// One voxelized object of the multi-object empty-space path.  Wherever the
-// ray lies in EMPTY cubes of a set of these objects (each on its own field)
-// and outside the balls of every other object (analytic or voxelized), each
-// object of the set samples its EMPTY value and every other object a larger
-// value, so the scene's minimum is the least EMPTY value of the set.
-constexpr uint32_t kMaxEmptyVox = 8;
-struct EmptyVox {
-  uint32_t obj;       // object index
-  uint32_t plain;     // zero translation and unit scale
-  float probe_min;    // probe for a cube once a sample was at least this
-  float empty_lo;     // lower bound of every EMPTY value (times the scale)
-  float empty_lo_t, empty_hi;  // tight bounds of an EMPTY step
-};
-
-struct KParams {
-  ObjDev objs[kMaxObjectsFast];  // object table in the constant parameter bank
-  SceneDev s;
-  const Segment* segs;
-  uint32_t nseg;
-  uint32_t tile_w, tile_h;
-  uint32_t interval;
-  uint64_t total;          // work ids of this launch: id0 .. id0 + total - 1
-  uint64_t id0;
-  unsigned long long* counter;
-  rkf_march_params p;
-  float probe_min;  // empty-space path: probe for a cube once a sample was at least this
-  uint32_t budget;     // empty-space path: steps per run before the warp re-converges
-  uint32_t plain_obj;  // object 0 has zero translation and unit scale
-  uint32_t refill_active;  // leave the march loop once at most this many lanes march
-  uint32_t run_probe;      // empty-space path: probe the next cube inside a run
-  uint32_t tail_share;     // empty-space path: warp-shared EMPTY runs once at most this many lanes march
-  TiledDev td;             // tiled strategy inputs (views of a tiled launch)
-  uint32_t tiled;
-  float empty_lo;          // empty-space path: lower bound of every EMPTY value
-  float empty_lo_t, empty_hi;  // empty-space path: tight bounds of an EMPTY step
-  uint32_t settle_links;   // empty-space path: cubes a settling chain may add (0 = off)
-  const rkf_bvh_node* bvh; // BVH strategy: the imported tree, root first
-  const uint32_t* bvh_next;  // per node: the walk's next node (bits 0-30), descend (bit 31)
-  uint32_t use_bvh;
-  // multi-object empty-space path: the voxelized objects that take EMPTY
-  // runs, and a ball for every object that needs one (bounding the largest
-  // EMPTY value of the path)
-  EmptyVox ev[kMaxEmptyVox];
-  uint32_t n_ev;
-  FarBall ball[kMaxObjectsFast];
-  uint32_t n_ball;
-};
-static_assert(sizeof(KParams) <= 32000, "the launch parameters must fit the kernel parameter space");
 
 // The candidate loop of ray_march_bvh (ray_march.wgsl:672-721): a stack walk
 // of the tree from the root that skips every node whose AABB lies farther
@@ -142,8 +77,9 @@ static_assert(sizeof(KParams) <= 32000, "the launch parameters must fit the kern
 // negative best).
 template <int PREC>
 __device__ __forceinline__ float eval_bvh(const SceneDev& s, const ObjDev* objs, const rkf_bvh_node* nodes,
-                                          const uint32_t* __restrict__ next, uint32_t nobj, float wx, float wy,
-                                          float wz, float& best_un, uint32_t& best_i, LaneCache& lc) {
+                                              const uint32_t* __restrict__ next, uint32_t nobj, float wx, float wy,
+                                              float wz, float& best_un, uint32_t& best_i) {
+  LaneCache lc;
   constexpr uint32_t kEnd = 0x7FFFFFFFu;
   float best = kMaxFloat;
   best_un = kMaxFloat;
@@ -184,278 +120,6 @@ __device__ __forceinline__ float eval_bvh(const SceneDev& s, const ObjDev* objs,
   return best;
 }
 
-// Object set of a launch: several objects, exactly one, or exactly one that
-// qualifies for the empty-space path (voxelized, translation-only
-// inverse_world, verified exact quotient, fewer than 2^20 voxels per axis).
-// OBJ_SINGLE_EMPTY_TILED: the empty-space path of a tiled launch (EMPTY runs
-// on the tiled empty-space field, tiled full steps elsewhere).
-// OBJ_MULTI_EMPTY: one object that qualifies for the empty-space path plus
-// analytic objects that each fit a ball (FarBall) and objects of no type; its
-// EMPTY runs and settling chains stay outside every ball.
-// OBJ_MULTI_EMPTY_TILED: the same under the tiled strategy (EMPTY runs on
-// the tiled empty-space field, for rays whose object list holds the
-// voxelized object; tiled full steps elsewhere).
-enum : int {
-  OBJ_MULTI = 0,
-  OBJ_SINGLE = 1,
-  OBJ_SINGLE_EMPTY = 2,
-  OBJ_SINGLE_EMPTY_TILED = 3,
-  OBJ_MULTI_EMPTY = 4,
-  OBJ_MULTI_EMPTY_TILED = 5
-};
-
-// Interval helpers in directed rounding: each result interval contains the
-// exact result for every value of the operand intervals.
-__device__ __forceinline__ void iv_mul(float x, float lo, float hi, float& rlo, float& rhi) {  // x * [lo, hi]
-  if (x >= 0.0f) {
-    rlo = __fmul_rd(x, lo);
-    rhi = __fmul_ru(x, hi);
-  } else {
-    rlo = __fmul_rd(x, hi);
-    rhi = __fmul_ru(x, lo);
-  }
-}
-__device__ __forceinline__ void iv_sq(float lo, float hi, float& rlo, float& rhi) {  // [lo, hi]^2
-  const float mlo = lo > 0.0f ? lo : (hi < 0.0f ? -hi : 0.0f);
-  const float mhi = fmaxf(fabsf(lo), fabsf(hi));
-  rlo = __fmul_rd(mlo, mlo);
-  rhi = __fmul_ru(mhi, mhi);
-}
-
-// Largest t' >= t such that every position of the ray o + d*u, u in [t, t'],
-// lies outside every ball (kMaxFloat when no ball lies ahead), skipping the
-// balls of the path objects in `skip` (those the run's set samples); -1 when the
-// position at t may lie inside one, with *recheck set to the earliest time
-// the ray may leave the balls that may hold it (else -1).  Per ball, with
-// w = o - c: the line's squared distance to the centre is |w|^2 - (d.w)^2/|d|^2,
-// its closest approach is at -(d.w)/|d|^2, and the chord within the ball
-// spans sqrt((rho^2 - h^2)/|d|^2) on each side.  Every quantity is an interval
-// evaluated in directed rounding, so the entry time used is a lower bound
-// and the exit time an upper bound of the exact ones.  A non-finite ray (or
-// a zero direction) makes every ball near.  Out of line: the march loop
-// calls it about once per ray, and its code would otherwise sit among the
-// loop's hot paths (measured 3% faster out of line).
-__device__ __noinline__ float far_limit(const FarBall* __restrict__ far, uint32_t n, uint32_t skip, float ox,
-                                           float oy, float oz, float dx, float dy, float dz, float tmax, float t,
-                                           float& recheck) {
-  const float a_lo = __fadd_rd(__fadd_rd(__fmul_rd(dx, dx), __fmul_rd(dy, dy)), __fmul_rd(dz, dz));
-  const float a_hi = __fadd_ru(__fadd_ru(__fmul_ru(dx, dx), __fmul_ru(dy, dy)), __fmul_ru(dz, dz));
-  // P >= |o| + |d| |tmax| (an L1 norm bounds the L2 norm)
-  const float P = __fadd_ru(__fadd_ru(__fadd_ru(fabsf(ox), fabsf(oy)), fabsf(oz)),
-                            __fmul_ru(__fsqrt_ru(a_hi), fabsf(tmax)));
-  float lim = kMaxFloat;
-  bool inside = false;
-  recheck = kMaxFloat;
-  for (uint32_t j = 0; j < n; ++j) {
-    const FarBall& f = far[j];
-    if (f.path < 32u && ((skip >> f.path) & 1u)) continue;  // an object of the run's set
-    if (f.box == 2) {
-      // half-space G.w + H <= m, m = a + b*P (a plane's small values lie in
-      // it): along the ray its coordinate G.(o + d u) + H - m is at least
-      // s0 + s1 u for u >= 0, both rounded down
-      const float m = __fadd_ru(f.a, __fmul_ru(f.b, P));
-      const float s0 = __fsub_rd(__fadd_rd(__fadd_rd(__fadd_rd(__fmul_rd(f.c[0], ox), __fmul_rd(f.c[1], oy)),
-                                                     __fmul_rd(f.c[2], oz)), f.h[0]), m);
-      const float s1 = __fadd_rd(__fadd_rd(__fmul_rd(f.c[0], dx), __fmul_rd(f.c[1], dy)), __fmul_rd(f.c[2], dz));
-      const float now = __fadd_rd(s0, __fmul_rd(s1, t));  // t >= 0
-      if (s1 >= 0.0f) {
-        if (now > 0.0f) continue;  // outside and not approaching: never inside
-        inside = true;             // may be inside now
-        // s0 <= now <= 0: outside again for u > -s0 / s1
-        if (s1 > 0.0f) recheck = fminf(recheck, __fdiv_ru(-s0, s1));
-      } else if (s1 < 0.0f && now > 0.0f) {
-        // approaching, outside now (s0 > 0): inside no earlier than s0 / -s1
-        lim = fminf(lim, fmaxf(t, __fdiv_rd(s0, -s1)));
-      } else {  // inside from now on, or NaN
-        inside = true;
-      }
-      continue;
-    }
-    if (f.box) {
-      // slab test of the box [c - h - m, c + h + m], m = a + b*P: the entry
-      // time rounded down and the exit time rounded up
-      const float m = __fadd_ru(f.a, __fmul_ru(f.b, P));
-      const float o3[3] = {ox, oy, oz}, d3[3] = {dx, dy, dz};
-      float e = -kMaxFloat, x = kMaxFloat;
-      bool miss = false;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float hw = __fadd_ru(f.h[k], m);
-        const float lo = __fsub_rd(f.c[k], hw), hi = __fadd_ru(f.c[k], hw);
-        if (d3[k] > 0.0f) {
-          e = fmaxf(e, __fdiv_rd(__fsub_rd(lo, o3[k]), d3[k]));
-          x = fminf(x, __fdiv_ru(__fsub_ru(hi, o3[k]), d3[k]));
-        } else if (d3[k] < 0.0f) {
-          e = fmaxf(e, __fdiv_rd(__fsub_ru(hi, o3[k]), d3[k]));
-          x = fminf(x, __fdiv_ru(__fsub_rd(lo, o3[k]), d3[k]));
-        } else if (!(o3[k] >= lo && o3[k] <= hi)) {
-          miss = true;  // parallel to this slab and outside it (NaN: not a miss)
-        }
-      }
-      if (miss || e > x) continue;
-      if (t < e) {
-        lim = fminf(lim, e);
-      } else if (!(t > x)) {  // may be inside now (or NaN)
-        inside = true;
-        recheck = fminf(recheck, x);
-      }
-      continue;
-    }
-    const float rho = __fadd_ru(f.a, __fmul_ru(f.b, P));
-    const float rho2 = __fmul_ru(rho, rho);
-    const float wxl = __fsub_rd(ox, f.c[0]), wxh = __fsub_ru(ox, f.c[0]);
-    const float wyl = __fsub_rd(oy, f.c[1]), wyh = __fsub_ru(oy, f.c[1]);
-    const float wzl = __fsub_rd(oz, f.c[2]), wzh = __fsub_ru(oz, f.c[2]);
-    float sxl, sxh, syl, syh, szl, szh;
-    iv_sq(wxl, wxh, sxl, sxh);
-    iv_sq(wyl, wyh, syl, syh);
-    iv_sq(wzl, wzh, szl, szh);
-    const float W_lo = __fadd_rd(__fadd_rd(sxl, syl), szl);
-    float pxl, pxh, pyl, pyh, pzl, pzh;  // d.w
-    iv_mul(dx, wxl, wxh, pxl, pxh);
-    iv_mul(dy, wyl, wyh, pyl, pyh);
-    iv_mul(dz, wzl, wzh, pzl, pzh);
-    const float b_lo = __fadd_rd(__fadd_rd(pxl, pyl), pzl), b_hi = __fadd_ru(__fadd_ru(pxh, pyh), pzh);
-    float b2l, b2h;
-    iv_sq(b_lo, b_hi, b2l, b2h);
-    const float h2_lo = __fsub_rd(W_lo, __fdiv_ru(b2h, a_lo));
-    if (h2_lo > rho2) continue;  // the line never comes within rho (NaN: not skipped)
-    const float half = __fsqrt_ru(__fdiv_ru(__fsub_ru(rho2, h2_lo), a_lo));
-    const float nb_lo = -b_hi, nb_hi = -b_lo;  // closest approach -(d.w)/|d|^2
-    const float tc_lo = __fdiv_rd(nb_lo, nb_lo < 0.0f ? a_lo : a_hi);
-    const float tc_hi = __fdiv_ru(nb_hi, nb_hi > 0.0f ? a_lo : a_hi);
-    const float e = __fsub_rd(tc_lo, half), x = __fadd_ru(tc_hi, half);
-    if (t < e) {
-      lim = fminf(lim, e);
-    } else if (!(t > x)) {  // may be inside now (or NaN)
-      inside = true;
-      recheck = fminf(recheck, x);
-    }
-  }
-  if (inside) return -1.0f;
-  recheck = -1.0f;
-  return lim;
-}
-
-// Grid coordinate (position + half grid size, object-local) of the ray at t,
-// rounded exactly as eval_obj -> sample_vox round it for a translation-only
-// object.
-__device__ __forceinline__ float grid_coord(float o, float d, float t, float m, float half) {
-  return __fadd_rn(__fadd_rn(__fadd_rn(o, __fmul_rn(d, t)), m), half);
-}
-
-// The EMPTY sampling value of sample_vox at a grid coordinate whose trilinear
-// cell lies in EMPTY blocks inside the grid and the geometry box (no clamp,
-// no outside term), times the object's scale: eval_obj's result there.
-__device__ __forceinline__ float empty_value(const ObjDev& o, float gx, float gy, float gz) {
-  const float vx = __fsub_rn(exact_div_vs(gx, o.vs, o.rcp_vs), 0.5f);
-  const float vy = __fsub_rn(exact_div_vs(gy, o.vs, o.rcp_vs), 0.5f);
-  const float vz = __fsub_rn(exact_div_vs(gz, o.vs, o.rcp_vs), 0.5f);
-  const float v = mix3_const(o.be, __fsub_rn(vx, floorf(vx)), __fsub_rn(vy, floorf(vy)), __fsub_rn(vz, floorf(vz)));
-  return __fmul_rn(v, o.min_scale);
-}
-
-// A ray as the EMPTY-cube probes see it: origin and step direction, the
-// direction's reciprocals (for the exit times) and the containment margin:
-// 0.1 voxel plus 2^-18 of the magnitudes involved, which covers every
-// rounding between t and the sampler's grid coordinate and every rounding of
-// the cube's faces and exit times computed here.
-struct ProbeRay {
-  float o[3], d[3], inv[3], margin;
-};
-
-__device__ __forceinline__ ProbeRay probe_ray(const ObjDev& ob, float ox, float oy, float oz, float dx, float dy,
-                                              float dz) {
-  ProbeRay r;
-  r.o[0] = ox, r.o[1] = oy, r.o[2] = oz;
-  r.d[0] = dx, r.d[1] = dy, r.d[2] = dz;
-  float mag = 1.0f;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    r.inv[a] = __frcp_rn(r.d[a]);
-    mag += fabsf(r.o[a]) + fabsf(ob.m[12 + a]) + ob.gs[a];
-  }
-  r.margin = 0.1f * ob.vs + mag * 3.814697265625e-6f;
-  return r;
-}
-
-// Largest t up to which the ray stays inside a cube of EMPTY blocks (from the
-// empty-space distance field), clipped to the grid and the geometry box, and
-// shrunk by the ray's margin: for each t' in [t_anchor, result] the trilinear
-// corners of the sample at t' lie in the cube, so the sample there is exactly
-// empty_value().  The cube is the one around the block of the position at
-// t_probe; which block that is only chooses the cube (its EMPTY-ness holds for
-// any block), so it is found with plain arithmetic, while the position at
-// t_anchor -- rounded exactly as the march rounds it -- must lie in the shrunk
-// cube.  Positions are monotone in t along each axis, so the exit faces
-// suffice.  -1 when there is no such cube.
-__device__ float probe_cube(const ObjDev& o, const uint8_t* __restrict__ field, const ProbeRay& r, float t_anchor,
-                            float t_probe) {
-  int k[3];
-  float p[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    p[a] = __fadd_rn(r.o[a], __fmul_rn(r.d[a], t_anchor));
-    const float pp = r.o[a] + r.d[a] * t_probe;
-    const float f = floorf((pp + o.m[12 + a] + o.half_gs[a]) * o.rcp_vs - 0.5f);
-    if (!(f >= 0.0f && f <= static_cast<float>(o.tv[a] - 1))) return -1.0f;
-    k[a] = static_cast<int>(f) >> 6;
-  }
-  const uint32_t s = __ldg(field + o.top_off + k[0] + k[1] * o.tdim[0] + k[2] * o.tdim[0] * o.tdim[1]);
-  if (s == 0) return -1.0f;
-  const int rad = static_cast<int>(s) - 1;  // every block within rad is EMPTY
-  float t_exit = kMaxFloat;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const int lo_v = max(0, (k[a] - rad) * 64), hi_v = min(o.tv[a] - 1, (k[a] + rad) * 64 + 63);
-    const float base = -o.half_gs[a] - o.m[12 + a];
-    float wlo = (static_cast<float>(lo_v) + 0.5f) * o.vs + base + r.margin;
-    float whi = (static_cast<float>(hi_v) + 0.5f) * o.vs + base - r.margin;
-    if (o.has_geom) {
-      wlo = fmaxf(wlo, o.gmin[a] - o.m[12 + a] + r.margin);
-      whi = fminf(whi, o.gmax[a] - o.m[12 + a] - r.margin);
-    }
-    if (!(p[a] >= wlo && p[a] <= whi)) return -1.0f;
-    if (r.d[a] > 0.0f) t_exit = fminf(t_exit, (whi - r.o[a]) * r.inv[a]);
-    else if (r.d[a] < 0.0f) t_exit = fminf(t_exit, (wlo - r.o[a]) * r.inv[a]);
-  }
-  return t_exit;
-}
-
-__device__ __forceinline__ float probe_empty(const ObjDev& o, const uint8_t* __restrict__ field, float ox,
-                                             float oy, float oz, float dx, float dy, float dz, float t) {
-  const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
-  return probe_cube(o, field, r, t, t);
-}
-
-// Extend an interval [t, cover] of EMPTY-cube positions along the ray through
-// at most `links` further cubes, until it reaches `need`.  The next cube is
-// the one around the block half a block ahead of the current end (else around
-// the end's own block) and must contain the current end, so the union stays
-// one interval.  Returns the new end.
-__device__ float extend_cover(const ObjDev& o, const uint8_t* __restrict__ field, float ox, float oy, float oz,
-                              float dx, float dy, float dz, float cover, float need, uint32_t links) {
-  const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
-  const float ahead = 32.0f * o.vs;
-  for (uint32_t i = 0; i < links && cover < need; ++i) {
-    float nx = probe_cube(o, field, r, cover, cover + ahead);
-    if (!(nx > cover)) {
-      nx = probe_cube(o, field, r, cover, cover);
-      if (!(nx > cover)) break;
-    }
-    cover = nx;
-  }
-  return cover;
-}
-
-__device__ __forceinline__ uint32_t find_segment(const Segment* segs, uint32_t nseg, uint64_t id) {
-  uint32_t lo = 0, hi = nseg;  // last segment with first <= id
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (segs[mid].first <= id) lo = mid; else hi = mid;
-  }
-  return lo;
-}
 
 // Minimum over objects [ob, oe) of evaluate_object at world position q.
 // SINGLE: the scene is exactly one object (object 0).
@@ -482,41 +146,28 @@ __device__ __forceinline__ float eval_min(const SceneDev& s, const ObjDev* objs,
   return best;
 }
 
-// Up to n march steps of a ray through EMPTY cubes: each sample is
-// empty_value().  The run stops before a step whose sample is below brk or
-// whose t is past tmax (the full step decides those), after the step that
-// makes max_near samples below near_thr, and where the ray leaves its cube
-// (t > box_t).  INRUN: a lane whose cube ends probes the next cube in place
-// and runs on (FAR: clipped at far_t, the end of the positions outside every
-// ball); stop_full tells whether the next step must be a full one.
+// Up to n march steps of a ray through positions covered by EMPTY boxes: each
+// sample is empty_value().  The run stops before a step whose sample is below
+// brk or whose t is past tmax (the full step decides those), after the step
+// that makes max_near samples below near_thr, and at the end of the covered
+// interval (t > box_t); stop_full tells whether the next step must be a full
+// one.
 // PLAIN: the object's translation is zero and its scale one, where adding the
-// translation and multiplying by the scale are exact identities.  CLEAN: every
-// EMPTY value is at least brk, near_thr and min_step (the caller checks this
-// against a lower bound), so those comparisons are known and skipped.
+// translation and multiplying by the scale are exact identities.
 // Returns the number of steps taken.
-template <bool PLAIN, bool CLEAN, bool INRUN, bool FAR>
-__device__ __forceinline__ uint32_t empty_run(const ObjDev& o, const uint8_t* __restrict__ field, float ox,
-                                              float oy, float oz, float dx, float dy, float dz, float tmax,
-                                              uint32_t n, float brk, float near_thr, float min_step,
-                                              uint32_t max_near, float far_t, float& t, float& box_t,
+template <bool PLAIN>
+__device__ __forceinline__ uint32_t empty_run(const ObjDev& o, float ox, float oy, float oz, float dx, float dy,
+                                              float dz, float tmax, uint32_t n, float brk, float near_thr,
+                                              float min_step, uint32_t max_near, float& t, float box_t,
                                               float& prev_t, float& prev_dist, uint32_t& near, bool& stop_full) {
   uint32_t c = 0;
-  float lim = fminf(box_t, tmax);
+  const float lim = fminf(box_t, tmax);
   stop_full = false;
 #pragma unroll 2
   for (; c < n; ++c) {
     if (t > lim) {
-      if (!INRUN || t > tmax) {
-        stop_full = t > tmax;
-        break;
-      }
-      box_t = probe_empty(o, field, ox, oy, oz, dx, dy, dz, t);
-      if (FAR) box_t = fminf(box_t, far_t);
-      lim = fminf(box_t, tmax);
-      if (t > lim) {
-        stop_full = true;
-        break;
-      }
+      stop_full = t > tmax;
+      break;
     }
     float gx, gy, gz;
     if (PLAIN) {
@@ -531,18 +182,14 @@ __device__ __forceinline__ uint32_t empty_run(const ObjDev& o, const uint8_t* __
     const float vx = __fsub_rn(exact_div_vs(gx, o.vs, o.rcp_vs), 0.5f);
     const float vy = __fsub_rn(exact_div_vs(gy, o.vs, o.rcp_vs), 0.5f);
     const float vz = __fsub_rn(exact_div_vs(gz, o.vs, o.rcp_vs), 0.5f);
-    float d = mix3_const(o.be, __fsub_rn(vx, floorf(vx)), __fsub_rn(vy, floorf(vy)), __fsub_rn(vz, floorf(vz)));
+    float d = mix3_const(o.be, frac_of(vx), frac_of(vy), frac_of(vz));
     if (!PLAIN) d = __fmul_rn(d, o.min_scale);
-    if (!CLEAN && !(d >= brk)) {  // no step: the full step redoes this sample
+    if (!(d >= brk)) {  // no step: the full step redoes this sample
       stop_full = true;
       break;
     }
     prev_t = t;
     prev_dist = d;
-    if (CLEAN) {
-      t = __fadd_rn(t, d);
-      continue;
-    }
     t = __fadd_rn(t, fmax_(d, min_step));
     if (d < near_thr && ++near >= max_near) {
       stop_full = true;
@@ -562,14 +209,15 @@ __device__ __forceinline__ float empty_value_x2(f2 o01, f2 d01, f2 h01, f2 r2, f
   const f2 q0 = f2_mul(g01, r2);
   const f2 v01 = f2_sub(f2_fma(f2_fma(q0, nvs2, g01), r2, q0), half2);
   const float vz = __fsub_rn(exact_div_vs(__fadd_rn(__fadd_rn(oz, __fmul_rn(dz, t)), hz), vs, rcp), 0.5f);
-  float vx, vy;
-  f2_unpack(v01, vx, vy);
+  const f2 magic = f2_pack(kIntMagic, kIntMagic);
   float tx, ty;
-  f2_unpack(f2_sub(v01, f2_pack(floorf(vx), floorf(vy))), tx, ty);
-  return mix3_const(be, tx, ty, __fsub_rn(vz, floorf(vz)));
+  f2_unpack(f2_sub(v01, f2_sub(f2_add(v01, magic), magic)), tx, ty);  // frac_of
+  return mix3_const(be, up_frac(tx), up_frac(ty), frac_of(vz));
 }
 
-// empty_run<PLAIN=true, CLEAN=true> two steps at a time.  Each step is
+// The run of a plain object whose every EMPTY value is at least brk, near_thr
+// and min_step (the caller checks this against a lower bound, so those
+// comparisons are known), two steps at a time.  Each step is
 // t' = t + E(t), a chain in which every step waits for the last.  E(t)
 // equals the brick extent c (the EMPTY constant) exactly for most positions
 // (the three nested mix(c, c, f) round back to c for about 93% of
@@ -577,34 +225,23 @@ __device__ __forceinline__ float empty_value_x2(f2 o01, f2 d01, f2 h01, f2 r2, f
 // rounding the step would make) and both E values are computed
 // independently.  The second step is accepted when the first value was
 // exactly c -- then its position is the one the serial march reaches, bit
-// for bit -- and when it passes the serial loop's checks (budget, cube end,
+// for bit -- and when it passes the serial loop's checks (budget, box end,
 // tmax); otherwise the first step is taken alone, with its value.  (Four
 // steps at a time measured 3-4% slower on the 1080p view: the longer code
 // raised instruction-fetch stalls by more than it cut dependency stalls.)
-template <bool INRUN, bool FAR>
-__device__ __forceinline__ uint32_t empty_run_x2(const ObjDev& o, const uint8_t* __restrict__ field, float ox,
-                                                 float oy, float oz, float dx, float dy, float dz, float tmax,
-                                                 uint32_t n, float far_t, float& t, float& box_t, float& prev_t,
-                                                 float& prev_dist, bool& stop_full) {
+__device__ __forceinline__ uint32_t empty_run_x2(const ObjDev& o, float ox, float oy, float oz, float dx, float dy,
+                                                 float dz, float tmax, uint32_t n, float& t, float box_t,
+                                                 float& prev_t, float& prev_dist, bool& stop_full) {
   uint32_t c = 0;
-  float lim = fminf(box_t, tmax);
+  const float lim = fminf(box_t, tmax);
   stop_full = false;
   const f2 o01 = f2_pack(ox, oy), d01 = f2_pack(dx, dy), h01 = f2_pack(o.half_gs[0], o.half_gs[1]);
   const f2 r2 = f2_pack(o.rcp_vs, o.rcp_vs), nvs2 = f2_pack(-o.vs, -o.vs), half2 = f2_pack(0.5f, 0.5f);
   const float hz = o.half_gs[2], vs = o.vs, rcp = o.rcp_vs, be = o.be;
   while (c < n) {
     if (t > lim) {
-      if (!INRUN || t > tmax) {
-        stop_full = t > tmax;
-        break;
-      }
-      box_t = probe_empty(o, field, ox, oy, oz, dx, dy, dz, t);
-      if (FAR) box_t = fminf(box_t, far_t);
-      lim = fminf(box_t, tmax);
-      if (t > lim) {
-        stop_full = true;
-        break;
-      }
+      stop_full = t > tmax;
+      break;
     }
     // the position of the next step if this value is c
     const float t1 = __fadd_rn(t, be);
@@ -624,76 +261,6 @@ __device__ __forceinline__ uint32_t empty_run_x2(const ObjDev& o, const uint8_t*
     t = __fadd_rn(pt, pd);
   }
   return c;
-}
-
-// empty_run_x2<INRUN=false>'s run taken by a whole warp, for the lanes that
-// pass pend, one lane's run after another (the launch's tail: few lanes
-// still march and the others have no work left).  Lane j of a round samples
-// the j-th step ahead.  Within t's binade [2^e, 2^(e+1)), whose spacing is u,
-// every t' is a multiple of u, so fl(t' + c) = t' + r with r = fl(t + c) - t
-// (c rounded to a multiple of u) unless c lies exactly halfway between two
-// multiples, where the rounding would depend on t' itself.  Away from such a
-// tie the serial positions while every value is c are therefore exactly
-// t + j*r (j*r and the sum are exact while t + j*r < 2^(e+1)), and lane j
-// computes its own without waiting for the others.  A round accepts the
-// steps up to the first value that is not c (that step is taken with its
-// value), or up to the first position past the binade, the run's end
-// (t > lim) or its budget (n steps), and the next position comes from the
-// last accepted step as the serial loop makes it.  A tie, or t too small
-// for this arithmetic, leaves lane 0 alone: one serial step per round.
-// Every lane of the warp must call this.
-__device__ __noinline__ void shared_runs(const ObjDev& o, bool pend, float ox, float oy, float oz, float dx,
-                                         float dy, float dz, float lim, float tmax, uint32_t n, float& t,
-                                         float& prev_t, float& prev_dist, uint32_t& c_out, bool& stop_full) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const f2 h01 = f2_pack(o.half_gs[0], o.half_gs[1]);
-  const f2 r2 = f2_pack(o.rcp_vs, o.rcp_vs), nvs2 = f2_pack(-o.vs, -o.vs), half2 = f2_pack(0.5f, 0.5f);
-  const float hz = o.half_gs[2], vs = o.vs, rcp = o.rcp_vs, be = o.be;
-  const float fj = static_cast<float>(lane);
-  for (uint32_t todo = __ballot_sync(kFull, pend); todo; todo &= todo - 1u) {
-    const uint32_t L = __ffs(todo) - 1u;
-    const float rox = __shfl_sync(kFull, ox, L), roy = __shfl_sync(kFull, oy, L), roz = __shfl_sync(kFull, oz, L);
-    const float rdx = __shfl_sync(kFull, dx, L), rdy = __shfl_sync(kFull, dy, L), rdz = __shfl_sync(kFull, dz, L);
-    const float rlim = __shfl_sync(kFull, lim, L), rtmax = __shfl_sync(kFull, tmax, L);
-    const uint32_t rn = __shfl_sync(kFull, n, L);
-    float rt = __shfl_sync(kFull, t, L);
-    const f2 o01 = f2_pack(rox, roy), d01 = f2_pack(rdx, rdy);
-    uint32_t c = 0;
-    float pt = 0.0f, pd = 0.0f;
-    bool sf = false;
-    for (;;) {
-      const uint32_t bits = __float_as_uint(rt) & 0x7f800000u;  // t >= 0
-      const float top = __uint_as_float(bits + 0x00800000u);    // 2^(e+1)
-      const float u = __uint_as_float(bits - (23u << 23));      // spacing of [2^e, 2^(e+1))
-      const float r = __fsub_rn(__fadd_rn(rt, be), rt);
-      const bool wide = rt >= 1.0e-30f && !(fabsf(__fsub_rn(be, r)) == __fmul_rn(0.5f, u));
-      const float tj = lane == 0 ? rt : __fadd_rn(rt, __fmul_rn(fj, r));
-      const bool ok = (lane == 0 || (wide && tj < top)) && !(tj > rlim) && c + lane < rn;
-      const float ej = empty_value_x2(o01, d01, h01, r2, nvs2, half2, roz, rdz, hz, vs, rcp, be, tj);
-      const uint32_t m_stop = __ballot_sync(kFull, !ok);
-      const uint32_t m_odd = __ballot_sync(kFull, ok && ej != be);
-      const uint32_t first_stop = m_stop ? __ffs(m_stop) - 1u : 32u;
-      const uint32_t first_odd = m_odd ? __ffs(m_odd) - 1u : 32u;
-      const uint32_t steps = first_odd < first_stop ? first_odd + 1u : first_stop;
-      if (steps == 0) {  // lane 0 stopped: the run ends here, as the serial loop ends it
-        sf = c < rn && rt > rtmax;
-        break;
-      }
-      pt = __shfl_sync(kFull, tj, steps - 1u);
-      pd = __shfl_sync(kFull, ej, steps - 1u);
-      c += steps;
-      rt = __fadd_rn(pt, pd);
-    }
-    if (lane == L) {
-      t = rt;
-      c_out = c;
-      stop_full = sf;
-      if (c) {
-        prev_t = pt;
-        prev_dist = pd;
-      }
-    }
-  }
 }
 
 // Up to n march steps through positions where every object of the set
@@ -748,6 +315,88 @@ __device__ __noinline__ uint32_t empty_run_set(const ObjDev* objs, const EmptyVo
 
 constexpr uint32_t kRefillRounds = 8;
 
+// What a hit's outputs are made of.
+struct HitRay {
+  float ox, oy, oz, rdx, rdy, rdz, t, mat_t, g0, g1, g2, sdf_hit;
+  uint32_t idx;
+  bool bisected, mat_ok;
+};
+
+// The G-buffer entry of a hit (ray_march.wgsl:1003-1032, :1068-1105).  Out of
+// line: few rays hit, and its divisions are a large part of a kernel's code.
+static __device__ __noinline__ void write_hit(const SceneDev& s, const ObjDev& o, const Segment& sg, const HitRay h) {
+  LaneCache lc;
+  const uint16_t flags = RKF_FLAG_HIT | (h.bisected ? RKF_FLAG_BISECTED : 0);
+  const float hx = __fadd_rn(h.ox, __fmul_rn(h.rdx, h.t)), hy = __fadd_rn(h.oy, __fmul_rn(h.rdy, h.t)),
+              hz = __fadd_rn(h.oz, __fmul_rn(h.rdz, h.t));
+  float gx = h.g0, gy = h.g1, gz = h.g2, sdf_hit = 0;
+  uint32_t slot = RKF_EMPTY_SLOT, mat = 0, sec = 0, blend = 0;
+  const bool vox = o.sdf_type == RKF_SDF_VOXELIZED;
+  if (vox) {
+    // world_grad = transpose(inverse_world) * (g, 0)  (:1014)
+    gx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[0], h.g0), __fmul_rn(o.m[1], h.g1)), __fmul_rn(o.m[2], h.g2)),
+                   __fmul_rn(o.m[3], 0.0f));
+    gy = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[4], h.g0), __fmul_rn(o.m[5], h.g1)), __fmul_rn(o.m[6], h.g2)),
+                   __fmul_rn(o.m[7], 0.0f));
+    gz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[8], h.g0), __fmul_rn(o.m[9], h.g1)), __fmul_rn(o.m[10], h.g2)),
+                   __fmul_rn(o.m[11], 0.0f));
+    float lpx, lpy, lpz;
+    to_local_fast(o, hx, hy, hz, lpx, lpy, lpz);
+    uint32_t vi = 0;
+    slot = nearest_slot(s, o, lpx, lpy, lpz, vi, lc);
+    if (slot < RKF_INTERIOR_SLOT) {
+      const size_t v = static_cast<size_t>(slot) * 512 + vi;
+      sec = (__ldg(s.mat + v) >> 6) & 0x3Fu;
+      blend = __ldg(s.blend + v);
+    }
+    sdf_hit = h.sdf_hit;  // taken when the motion plane is asked for
+  }
+  const float l = len3(gx, gy, gz);
+  float nx = 0, ny = 1.0f, nz = 0;
+  if (!(vox && l < 1e-10f)) {
+    nx = __fdiv_rn(gx, l);
+    ny = __fdiv_rn(gy, l);
+    nz = __fdiv_rn(gz, l);
+  }
+  if (h.mat_ok || o.sdf_type == RKF_SDF_ANALYTICAL)
+    mat = material_at(s, o, __fadd_rn(h.ox, __fmul_rn(safe_dir(h.rdx), h.mat_t)),
+                      __fadd_rn(h.oy, __fmul_rn(safe_dir(h.rdy), h.mat_t)),
+                      __fadd_rn(h.oz, __fmul_rn(safe_dir(h.rdz), h.mat_t)), lc);
+  const size_t i = h.idx;
+  sg.t[i] = h.t;
+  if (sg.normal) {
+    sg.normal[3 * i] = nx;
+    sg.normal[3 * i + 1] = ny;
+    sg.normal[3 * i + 2] = nz;
+  }
+  if (sg.slot) sg.slot[i] = slot;
+  if (sg.material) sg.material[i] = static_cast<uint16_t>(mat);
+  if (sg.flags) sg.flags[i] = flags;
+  if (sg.position) reinterpret_cast<float4*>(sg.position)[i] = make_float4(hx, hy, hz, h.t);
+  if (sg.packed) sg.packed[i] = (mat & 0x3Fu) | (sec << 6) | (blend << 12) | (o.object_id << 24);
+  if (sg.motion) {
+    const float* m = sg.prev_vp;  // ray_march.wgsl:1094-1105
+    const float cx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], hx), __fmul_rn(m[4], hy)), __fmul_rn(m[8], hz)),
+                               __fmul_rn(m[12], 1.0f));
+    const float cy = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[1], hx), __fmul_rn(m[5], hy)), __fmul_rn(m[9], hz)),
+                               __fmul_rn(m[13], 1.0f));
+    const float cw = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[3], hx), __fmul_rn(m[7], hy)), __fmul_rn(m[11], hz)),
+                               __fmul_rn(m[15], 1.0f));
+    float mox = 0.f, moy = 0.f;
+    if (cw > 0.0f) {
+      const float ndx = __fdiv_rn(cx, cw), ndy = __fdiv_rn(cy, cw);
+      const float pu = __fadd_rn(__fmul_rn(ndx, 0.5f), 0.5f);
+      const float pv = __fsub_rn(0.5f, __fmul_rn(ndy, 0.5f));
+      const uint32_t px = h.idx % sg.w, py = h.idx / sg.w;
+      const float cu = __fdiv_rn(__fadd_rn(static_cast<float>(px), 0.5f), static_cast<float>(sg.w));
+      const float cv = __fdiv_rn(__fadd_rn(static_cast<float>(py), 0.5f), static_cast<float>(sg.h));
+      mox = __fsub_rn(cu, pu);
+      moy = __fsub_rn(cv, pv);
+    }
+    reinterpret_cast<float4*>(sg.motion)[i] = make_float4(mox, moy, 1.0f, sdf_hit);
+  }
+}
+
 // The outputs of a ray that ends at its first check, unhit, with no step
 // taken (its tmax is below its starting t): what the epilogue writes for it.
 __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, uint32_t mode,
@@ -758,31 +407,64 @@ __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, ui
     return;
   }
   const uint16_t flags = (0u >= p.hard_max_steps || 0u >= p.scene.max_steps) ? RKF_FLAG_STEPS_OUT : 0;
-  sg.t[idx] = kMaxFloat;
-  if (sg.flags) sg.flags[idx] = flags;
-  if (mode == RKF_TRACE_ANY) return;
-  if (sg.normal) {
-    sg.normal[3 * static_cast<size_t>(idx)] = 0.0f;
-    sg.normal[3 * static_cast<size_t>(idx) + 1] = 0.0f;
-    sg.normal[3 * static_cast<size_t>(idx) + 2] = 0.0f;
+  if (mode == RKF_TRACE_ANY) {
+    sg.t[idx] = kMaxFloat;
+    if (sg.flags) sg.flags[idx] = flags;
+    return;
   }
-  if (sg.slot) sg.slot[idx] = RKF_EMPTY_SLOT;
-  if (sg.material) sg.material[idx] = 0;
-  if (sg.position) reinterpret_cast<float4*>(sg.position)[idx] = make_float4(0.f, 0.f, 0.f, kMaxFloat);
-  if (sg.packed) sg.packed[idx] = 0u;
-  if (sg.motion) reinterpret_cast<float4*>(sg.motion)[idx] = make_float4(0.f, 0.f, 0.f, 0.f);
+  write_miss(sg, idx, flags);
+}
+
+// The march kernel is bound by issue slots and by instruction fetch: its lanes
+// are in different phases of their rays (walking ahead, running over EMPTY
+// samples, evaluating a sample, done), what one lane does the other lanes of
+// its warp wait for, and every phase's code has to come through the
+// instruction cache.  So a warp takes one phase at a time, the one that most of
+// its lanes are ready for, and hands out new rays as soon as kRefillLanes of its
+// lanes are done.  All samples of a ray -- its steps, its bisection, its normal
+// -- go through the one evaluation phase, so the kernel holds one copy of the
+// sampler: 76 KB of code instead of 209 KB.  1920x1080 over the 1.1M-brick
+// scene: 1.45 ms for the kernel that took the phases in lockstep, 0.99 ms with
+// the settling passes (settle.cu) before this one.
+//
+// Measured choices (us: that view / 960x540 of the same scene / 4 views of it
+// with their shadow and occlusion rays / 256x256, f32, of the 32 m scene):
+//   new rays at 16 lanes done 990 / 605 / 3,300 / 417, at 20 986 / 601 / 3,286 /
+//   412, at 24 989 / 596 / 3,235 / 413; waiting for all 32: 1,390 and more.
+//   3 blocks an SM 986 / 601 / 3,286 / 412, 4 (64 registers, which spill)
+//   1,062 / 659 / 3,112 / 431, 2 1,007 / 547 / 3,659 / 432.
+//   A walk that brought no run of kShortRun EMPTY steps puts the next one off by
+//   kPutOff: 8 and 8 1,069 / 659 / 3,165 / 426, no putting off 1,157 / 675 /
+//   3,691 / 425, 16 and 16 1,092 / 654 / 3,173 / 432 (with 4 blocks).
+// The variants of several objects and of the tiled strategy hold more state: 2
+// blocks (1277x717, the 1.1M-brick scene and four more objects: 1.42 ms against
+// 1.49 with 4), and their plain kin stay at 4 (u8, 1920x1080 of the 32 m scene:
+// 1.64 ms against 1.85 with 5 and 1.73 with 3).
+constexpr uint32_t kRefillLanes = 24;
+constexpr float kShortRun = 8.0f, kPutOff = 8.0f;  // in EMPTY steps
+constexpr uint32_t kWalkLinks = 64;   // boxes a walk takes in one phase
+constexpr uint32_t kLeastLanes = 4;   // lanes a warp fills however few rays there are
+constexpr uint32_t kEvalReps = 8;     // samples a lane takes in one phase
+constexpr int march_blocks(int obj) { return obj >= OBJ_SINGLE_EMPTY_TILED ? 2 : obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
+constexpr uint32_t march_refill(int obj) { return obj == OBJ_MULTI || obj == OBJ_SINGLE ? 16u : kRefillLanes; }
+#define kNoBox __int_as_float(0x7fc00000)  // compares false with every time
+
+// A warp's lanes' share of the ids left to hand out.
+__device__ __forceinline__ uint32_t lane_share(uint64_t total, uint64_t handed, uint32_t warps) {
+  const uint64_t left = total > handed ? total - handed : 0u;
+  if (left >= static_cast<uint64_t>(warps) * 32u) return 32u;
+  return max((static_cast<uint32_t>(left) + warps - 1u) / warps, kLeastLanes);
 }
 
 template <int PREC, int OBJ>
-__global__ void __launch_bounds__(256, 4) k_march_persistent(const __grid_constant__ KParams kp) {
+__global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(const __grid_constant__ KParams kp) {
   constexpr bool MULTI_TILED = OBJ == OBJ_MULTI_EMPTY_TILED;
   constexpr bool MULTI_EMPTY = OBJ == OBJ_MULTI_EMPTY || MULTI_TILED;
   constexpr bool SINGLE = OBJ != OBJ_MULTI && !MULTI_EMPTY;
   constexpr bool EMPTY_PATH = OBJ == OBJ_SINGLE_EMPTY || OBJ == OBJ_SINGLE_EMPTY_TILED || MULTI_EMPTY;
+  constexpr bool PLAIN_VOX = OBJ == OBJ_SINGLE_EMPTY || OBJ == OBJ_SINGLE_EMPTY_TILED;
   // tile bookkeeping of tiled launches
   constexpr bool TILES = OBJ != OBJ_SINGLE_EMPTY && OBJ != OBJ_MULTI_EMPTY;
-  // warp-shared EMPTY runs in the launch's tail (shared_runs)
-  constexpr bool SHARE = OBJ == OBJ_SINGLE_EMPTY;
   // the object table: the launch parameters hold up to kMaxObjectsFast
   // records; a larger scene (the plain multi-object variant only) reads the
   // device copy
@@ -802,585 +484,602 @@ __global__ void __launch_bounds__(256, 4) k_march_persistent(const __grid_consta
   ColdState& cs = cold_all[threadIdx.x];
   float ox = 0, oy = 0, oz = 0, rdx = 0, rdy = 0, rdz = 0;
   float t = 0, prev_t = 0, prev_dist = kMaxFloat, tmax = 0;
-  float box_t = -1.0f;  // empty-space path: positions up to here sample the EMPTY value
-  float far_t = -1.0f;  // multi-object empty-space path: positions up to here lie outside every ball
-  float far_recheck = -1.0f;  // multi-object empty-space path: no ball check before this t
+  // empty-space path: positions up to here sample the EMPTY value (kNoBox: none;
+  // negative: a walk goes on)
+  float box_t = kNoBox;
+  float far_t = -1.0f;   // multi-object empty-space path: positions up to here lie outside every ball
+  float probe_t = 0.0f;  // empty-space path: no walk before this t
   uint32_t near = 0, step = 0;
+  uint32_t since = 0;  // phases since the warp last took new rays
+  // Lanes a warp fills: all of them while there is work for every warp's, else
+  // its share of what is left, so that a small launch, and the end of a large
+  // one, spreads its rays over the chip's warps instead of packing 32 rays in
+  // different phases into each of a few.
+  const uint32_t n_list = kp.list ? __ldg(kp.list_n) : 0u;
+  const uint64_t total = kp.list ? kp.total - kp.view_ids + n_list : kp.total;
+  uint32_t lanes = lane_share(total, 0, gridDim.x * (blockDim.x >> 5));
   bool exhausted = false;
 
   for (;;) {
-    // ---- 1. refill idle lanes ------------------------------------------------
-    // A ray that ends before its first sample (tmax below its starting t:
-    // the secondary rays of pixels that missed) takes its outputs here and
-    // its lane takes the next id at once, for up to kRefillRounds rounds, so
-    // that such rays do not leave lanes idle through the march loop.
-    for (uint32_t round = 0; round < kRefillRounds; ++round) {
-      const bool idle = state == ST_IDLE;
-      const uint32_t need = __ballot_sync(kFull, idle);
-      bool again = false;  // this lane's id ended at once (or is off the view)
-      if (need && !exhausted) {
-        const uint32_t leader = __ffs(need) - 1;
-        unsigned long long base = 0;
-        if (lane == leader) base = atomicAdd(kp.counter, static_cast<unsigned long long>(__popc(need)));
-        base = __shfl_sync(kFull, base, leader);
-        if (base + __popc(need) >= kp.total) exhausted = true;
-        if (idle) {
-          const uint64_t k = base + __popc(need & ((1u << lane) - 1u));
-          if (k < kp.total) {
-            const uint64_t id = kp.id0 + k;
-            cs.seg = find_segment(kp.segs, kp.nseg, id);
-            const Segment& sg = kp.segs[cs.seg];
-            const uint64_t local = id - sg.first;
-            bool valid = true;
-            if (sg.kind == 0) {  // view: tile-ordered pixel ids
-              const uint32_t per = kp.tile_w * kp.tile_h;
-              uint32_t tile = static_cast<uint32_t>(local / per);
-              if (sg.tile_perm) tile = __ldg(sg.tile_perm + tile);  // heaviest-first order
-              const uint32_t r = static_cast<uint32_t>(local % per);
-              const uint32_t px = (tile % sg.tiles_x) * kp.tile_w + r % kp.tile_w;
-              const uint32_t py = (tile / sg.tiles_x) * kp.tile_h + r / kp.tile_w;
-              valid = px < sg.w && py < sg.h;
-              if (valid) {
-                cs.idx = py * sg.w + px;
-                // ray generation (ray_march.wgsl:1046-1053)
-                const float u = __fdiv_rn(__fadd_rn(__fadd_rn(static_cast<float>(px), 0.5f), sg.jitter[0]),
-                                          static_cast<float>(sg.w));
-                const float v = __fdiv_rn(__fadd_rn(__fadd_rn(static_cast<float>(py), 0.5f), sg.jitter[1]),
-                                          static_cast<float>(sg.h));
-                const float nx = __fsub_rn(__fmul_rn(u, 2.0f), 1.0f);
-                const float ny = __fsub_rn(1.0f, __fmul_rn(v, 2.0f));
-                const float vx = __fadd_rn(__fadd_rn(sg.fwd[0], __fmul_rn(sg.right[0], nx)), __fmul_rn(sg.up[0], ny));
-                const float vy = __fadd_rn(__fadd_rn(sg.fwd[1], __fmul_rn(sg.right[1], nx)), __fmul_rn(sg.up[1], ny));
-                const float vz = __fadd_rn(__fadd_rn(sg.fwd[2], __fmul_rn(sg.right[2], nx)), __fmul_rn(sg.up[2], ny));
-                const float l = len3(vx, vy, vz);
-                rdx = __fdiv_rn(vx, l);
-                rdy = __fdiv_rn(vy, l);
-                rdz = __fdiv_rn(vz, l);
-                ox = sg.pos[0];
-                oy = sg.pos[1];
-                oz = sg.pos[2];
-                tmax = p.scene.max_distance;
-                mode = RKF_TRACE_CLOSEST;
-                if (TILES) {
-                  cs.tile_count = kNoTiles;
-                  if (kp.tiled) {  // the pixel's tile (ray_march.wgsl:884-893)
-                    const uint32_t tl = sg.tile_off + (py / 16) * ((sg.w + 15) / 16) + px / 16;
-                    cs.tile_base = tl * kTileObjects;
-                    cs.tile_count = __ldg(kp.td.tile_cnt + tl);
-                  }
-                  if (MULTI_TILED) {
-                    uint32_t listed = 0;
-                    for (uint32_t e = 0; e < kp.n_ev; ++e) {
-                      bool in = cs.tile_count == kNoTiles;
-                      for (uint32_t j = 0; !in && j < cs.tile_count; ++j)
-                        in = __ldg(kp.td.tile_list + cs.tile_base + j) == kp.ev[e].obj;
-                      if (in) listed |= 1u << e;
+    const bool march = state == ST_MARCH || state == ST_SHADOW;
+    // the march steps along the safe direction (ray_march.wgsl:784); hit
+    // positions use the raw direction (:1068), as shadow rays do
+    const bool sh = state == ST_SHADOW;
+    const float dx = sh ? rdx : safe_dir(rdx), dy = sh ? rdy : safe_dir(rdy), dz = sh ? rdz : safe_dir(rdz);
+    // what ends a ray, and what its samples are compared with: a sample below
+    // brk is decided by the evaluation phase
+    const uint32_t max_step = sh ? 256u : p.hard_max_steps;
+    const uint32_t max_near = sh ? 32u : p.scene.max_steps;
+    const float brk = sh ? 0.02f : fmaxf(hit_thr, 0.0f);
+    const float near_thr = sh ? -1.0f : p.near_surface_threshold;
+    const float min_step = sh ? 0.005f : p.min_step;
+
+    // ---- the phase most lanes are ready for -----------------------------------
+    const bool run = EMPTY_PATH && march && t <= box_t;
+    const bool walk = EMPTY_PATH && march && !run && (box_t < 0.0f || (t >= probe_t && prev_dist >= kp.probe_min));
+    const bool done = state == ST_IDLE || state == ST_EPI;
+    const uint32_t n_done = __popc(__ballot_sync(kFull, done));
+    const uint32_t n_walk = EMPTY_PATH ? __popc(__ballot_sync(kFull, walk)) : 0u;
+    const uint32_t n_run = EMPTY_PATH ? __popc(__ballot_sync(kFull, run)) : 0u;
+    const uint32_t n_eval = 32u - n_done - n_walk - n_run;
+    ++since;
+
+    if (n_done == 32u || (!exhausted && (n_done >= kp.refill_idle + 32u - lanes ||
+                                         (n_done > 32u - lanes && since >= kp.interval)))) {
+      // ---- outputs of finished rays --------------------------------------------
+      if (state == ST_EPI) {
+        const Segment& sg = kp.segs[cs.seg];
+        if (mode == RKF_TRACE_SHADOW) {
+          sg.t[cs.idx] = clampf(cs.shadow, 0.0f, 1.0f);
+          if (sg.flags) sg.flags[cs.idx] = cs.hit ? RKF_FLAG_HIT : 0;
+        } else if (mode == RKF_TRACE_ANY) {
+          sg.t[cs.idx] = cs.hit ? t : kMaxFloat;
+          if (sg.flags)
+            sg.flags[cs.idx] = cs.hit ? RKF_FLAG_HIT
+                                : ((step >= p.hard_max_steps || near >= p.scene.max_steps) ? RKF_FLAG_STEPS_OUT : 0);
+        } else {
+          if (!cs.hit) {
+            write_miss(sg, cs.idx,
+                       step >= p.hard_max_steps || near >= p.scene.max_steps ? RKF_FLAG_STEPS_OUT : uint16_t(0));
+          } else {
+            const HitRay h{ox, oy, oz, rdx, rdy, rdz, t, cs.mat_t, cs.g[0], cs.g[1], cs.g[2], cs.sdf_hit,
+                           cs.idx, cs.bisected, cs.mat_ok};
+            write_hit(s, sh_objs[cs.hit_obj], sg, h);
+          }
+        }
+        state = ST_IDLE;
+      }
+      if (exhausted) break;  // every lane is done and no work is left
+      since = 0;
+      // ---- new rays for the idle lanes -------------------------------------------
+      // A ray that ends before its first sample (tmax below its starting t:
+      // the secondary rays of pixels that missed) takes its outputs here and
+      // its lane takes the next id at once, for up to kRefillRounds rounds, so
+      // that such rays do not leave lanes idle through the march loop.
+      for (uint32_t round = 0; round < kRefillRounds; ++round) {
+        const bool idle = state == ST_IDLE;
+        uint32_t need = __ballot_sync(kFull, idle);
+        // (the first of the idle lanes, up to the warp's share)
+        const uint32_t busy = 32u - __popc(need);
+        const uint32_t room = lanes > busy ? lanes - busy : 0u;
+        const bool take = idle && __popc(need & ((1u << lane) - 1u)) < room;
+        need = __ballot_sync(kFull, take);
+        bool again = false;  // this lane's id ended at once (or is off the view)
+        if (need && !exhausted) {
+          const uint32_t leader = __ffs(need) - 1;
+          unsigned long long base = 0;
+          if (lane == leader) base = atomicAdd(kp.counter, static_cast<unsigned long long>(__popc(need)));
+          base = __shfl_sync(kFull, base, leader);
+          if (base + __popc(need) >= total) exhausted = true;
+          lanes = lane_share(total, base + __popc(need), gridDim.x * (blockDim.x >> 5));
+          if (take) {
+            const uint64_t k = base + __popc(need & ((1u << lane) - 1u));
+            if (k < total) {
+              // the rays the settling passes left, then the ray batches
+              const bool listed = kp.list && k < n_list;
+              const uint2 entry = listed ? __ldg(kp.list + k) : make_uint2(0u, 0x7fc00000u);
+              const uint64_t id = listed ? entry.x : kp.list ? kp.view_ids + (k - n_list) : kp.id0 + k;
+              cs.seg = find_segment(kp.segs, kp.nseg, id);
+              const Segment& sg = kp.segs[cs.seg];
+              const uint64_t local = id - sg.first;
+              bool valid = true;
+              if (sg.kind == 0) {  // view: tile-ordered pixel ids
+                const uint32_t per = kp.tile_w * kp.tile_h;
+                // (32-bit division where the view's ids fit it)
+                uint32_t tile = (sg.n_ids >> 32) ? static_cast<uint32_t>(local / per) : static_cast<uint32_t>(local) / per;
+                const uint32_t r = static_cast<uint32_t>(local - static_cast<uint64_t>(tile) * per);
+                if (sg.tile_perm) tile = __ldg(sg.tile_perm + tile);  // heaviest-first order
+                const uint32_t px = (tile % sg.tiles_x) * kp.tile_w + r % kp.tile_w;
+                const uint32_t py = (tile / sg.tiles_x) * kp.tile_h + r / kp.tile_w;
+                valid = px < sg.w && py < sg.h;
+                if (valid) {
+                  cs.idx = py * sg.w + px;
+                  view_ray(sg, px, py, rdx, rdy, rdz);
+                  ox = sg.pos[0];
+                  oy = sg.pos[1];
+                  oz = sg.pos[2];
+                  tmax = p.scene.max_distance;
+                  mode = RKF_TRACE_CLOSEST;
+                  if (TILES) {
+                    cs.tile_count = kNoTiles;
+                    if (kp.tiled) {  // the pixel's tile (ray_march.wgsl:884-893)
+                      const uint32_t tl = sg.tile_off + (py / 16) * ((sg.w + 15) / 16) + px / 16;
+                      cs.tile_base = tl * kTileObjects;
+                      cs.tile_count = __ldg(kp.td.tile_cnt + tl);
                     }
-                    cs.vox_listed = listed;
+                    if (MULTI_TILED) {
+                      uint32_t listed = 0;
+                      for (uint32_t e = 0; e < kp.n_ev; ++e) {
+                        bool in = cs.tile_count == kNoTiles;
+                        for (uint32_t j = 0; !in && j < cs.tile_count; ++j)
+                          in = __ldg(kp.td.tile_list + cs.tile_base + j) == kp.ev[e].obj;
+                        if (in) listed |= 1u << e;
+                      }
+                      cs.vox_listed = listed;
+                    }
                   }
                 }
-              }
-            } else {
-              if (TILES) cs.tile_count = kNoTiles;
-              if (MULTI_TILED) cs.vox_listed = (1u << kp.n_ev) - 1u;
-              cs.idx = static_cast<uint32_t>(local);
-              const size_t i3 = 3 * static_cast<size_t>(cs.idx);
-              ox = __ldg(sg.origins + i3);
-              oy = __ldg(sg.origins + i3 + 1);
-              oz = __ldg(sg.origins + i3 + 2);
-              rdx = __ldg(sg.dirs + i3);
-              rdy = __ldg(sg.dirs + i3 + 1);
-              rdz = __ldg(sg.dirs + i3 + 2);
-              tmax = __ldg(sg.tmax + cs.idx);
-              mode = sg.mode;
-            }
-            if (valid) {
-              near = 0;
-              step = 0;
-              box_t = -1.0f;
-              if (MULTI_EMPTY) {
-                far_t = far_recheck = -1.0f;
-                if (!MULTI_TILED) cs.vox_listed = (1u << kp.n_ev) - 1u;
-              }
-              prev_dist = kMaxFloat;
-              cs.hit = cs.bisected = cs.mat_ok = false;
-              if (mode == RKF_TRACE_SHADOW) {
-                t = 0.005f;  // SHADOW_EPSILON (shade_common.wgsl:274)
-                cs.shadow = 1.0f;
-                state = ST_SHADOW;
               } else {
-                t = 0.0f;
-                prev_t = 0.0f;
-                prev_dist = kMaxFloat;
-                // a tile with no objects is sky (ray_march.wgsl:895-897)
-                state = (TILES && cs.tile_count == 0) ? ST_EPI : ST_MARCH;
+                if (TILES) cs.tile_count = kNoTiles;
+                if (MULTI_TILED) cs.vox_listed = (1u << kp.n_ev) - 1u;
+                cs.idx = static_cast<uint32_t>(local);
+                const size_t i3 = 3 * static_cast<size_t>(cs.idx);
+                tmax = __ldg(sg.tmax + cs.idx);
+                mode = sg.mode;
+                ox = __ldg(sg.origins + i3);
+                oy = __ldg(sg.origins + i3 + 1);
+                oz = __ldg(sg.origins + i3 + 2);
+                rdx = __ldg(sg.dirs + i3);
+                rdy = __ldg(sg.dirs + i3 + 1);
+                rdz = __ldg(sg.dirs + i3 + 2);
               }
-              if (state != ST_EPI && t > tmax) {
-                // its first check ends it unhit with no step taken: the
-                // epilogue's outputs for that (shadow 1; t max, normal 0,
-                // EMPTY slot, material 0, STEPS_OUT only when the near-step
-                // limit is 0, the miss position and motion)
-                write_unmarched(sg, cs.idx, mode, p);
-                state = ST_IDLE;
+              if (valid) {
+                near = 0;
+                step = 0;
+                box_t = __uint_as_float(entry.y);  // how far the settling pass saw EMPTY samples
+                probe_t = box_t == box_t ? after(0.0f) : 0.0f;
+                if (MULTI_EMPTY) {
+                  far_t = -1.0f;
+                  // (the normal's until then: no settling attempt before this t,
+                  // and the first ball ahead)
+                  cs.gpos = box_t == box_t ? box_t : 0.0f;
+                  cs.g[0] = -1.0f;
+                  cs.g[1] = 2.0f * kp.empty_hi;
+                  box_t = kNoBox;
+                  probe_t = 0.0f;
+                  if (!MULTI_TILED) cs.vox_listed = (1u << kp.n_ev) - 1u;
+                }
+                prev_dist = kMaxFloat;
+                cs.hit = cs.bisected = cs.mat_ok = false;
+                if (mode == RKF_TRACE_SHADOW) {
+                  t = 0.005f;  // SHADOW_EPSILON (shade_common.wgsl:274)
+                  cs.shadow = 1.0f;
+                  state = ST_SHADOW;
+                } else {
+                  t = 0.0f;
+                  prev_t = 0.0f;
+                  // a tile with no objects is sky (ray_march.wgsl:895-897); a
+                  // step limit of 0 ends the ray at its first check
+                  state = ((TILES && cs.tile_count == 0) || p.scene.max_steps == 0 || p.hard_max_steps == 0)
+                              ? ST_EPI : ST_MARCH;
+                }
+                if (state != ST_EPI && t > tmax) {
+                  // its first check ends it unhit with no step taken: the
+                  // epilogue's outputs for that (shadow 1; t max, normal 0,
+                  // EMPTY slot, material 0, the miss position and motion)
+                  write_unmarched(sg, cs.idx, mode, p);
+                  state = ST_IDLE;
+                  again = true;
+                }
+              } else {
                 again = true;
               }
-            } else {
-              again = true;
             }
           }
         }
+        if (!__any_sync(kFull, again)) break;
       }
-      if (!__any_sync(kFull, again)) break;
-    }
-    if (__all_sync(kFull, state == ST_IDLE)) {
-      if (exhausted) break;
       continue;
     }
-    // the march steps along the safe direction (ray_march.wgsl:784); cs.hit
-    // positions use the raw direction (:1068)
-    const float qdx = fabsf(rdx) < 1e-10f ? 1e-10f : rdx;
-    const float qdy = fabsf(rdy) < 1e-10f ? 1e-10f : rdy;
-    const float qdz = fabsf(rdz) < 1e-10f ? 1e-10f : rdz;
 
-    // ---- 2. tight march loop -------------------------------------------------
+    if (EMPTY_PATH && n_walk && n_walk >= n_run && n_walk >= n_eval) {
+      // ---- walk: where the samples ahead are known to be EMPTY -------------------
+      // A lane whose last sample was (close to) the EMPTY value walks its ray
+      // ahead through EMPTY boxes.  If every sample the ray has left is at
+      // least the EMPTY value and that clears every threshold, no decision is
+      // left to take: the ray misses, its outputs do not depend on its exact t,
+      // and it is settled here.  Otherwise the walk's end bounds the run.
+      if (walk) {
+        uint32_t outcome = 0;  // 1: ends past tmax; 2: runs out of steps
+        // t after k more steps lies in [t + k*lo, t + k*hi] widened by one
+        // rounding (2^-24) per step; 2^-22 per step (and 4 more) leaves room
+        // for this bound's own rounding.  The last sample is the
+        // (max_step-step-1)th ahead: the ray ends past tmax (with no step
+        // flag) if even its smallest t exceeds tmax by then, and runs out of
+        // steps if even its largest t stays <= tmax.
+        const float k = static_cast<float>(max_step - step - 1);
+        const float grow = (k + 4.0f) * 2.384185791015625e-7f;
+        const float t_lo = (t + k * kp.empty_lo_t) * (1.0f - grow);
+        const float t_hi = (t + k * kp.empty_hi) * (1.0f + grow);
+        const bool can = kp.empty_lo >= brk && kp.empty_lo >= near_thr && kp.empty_lo >= min_step;
+        if (!MULTI_EMPTY) {
+          // A walk takes kWalkLinks boxes a phase and goes on in the next, so
+          // that lanes that are done make room for new rays meanwhile.  While a
+          // walk goes on, box_t is minus its end, probe_t its target, and the
+          // rest of its state in the cold one.
+          const ObjDev& o = sh_objs[0];
+          const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
+          float end = -1.0f, out[3];
+          bool more = true;
+          if (box_t < 0.0f) {
+            end = -box_t;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) out[a] = cs.g[a];
+          } else {
+            float t_in, t_out;
+            const bool core = core_interval(o, r, t, t_in, t_out);
+            float target = core ? t_out : -1.0f;
+            if (can) {
+              if (t_lo > tmax) {
+                outcome = 1;
+                target = tmax;
+              } else if (t_hi <= tmax && core && t_out >= t_hi) {
+                outcome = 2;
+                target = t_hi;
+              } else if (OBJ == OBJ_SINGLE_EMPTY) {
+                outcome = leaves_grid(o, r, t, tmax, core, t_out, k, kp.empty_lo_t, kp.empty_hi);
+                if (outcome) target = tmax;
+              }
+            }
+            cs.vox_listed = outcome;
+            cs.hi = core ? t_out : -1.0f;  // (the bisection's until then)
+            // outside: nothing to walk for before the ray enters
+            cs.lo = core || (t_in < t_out && t < t_out && !(t_in > t)) ? after(t)
+                    : t_in < t_out && t_in > t ? t_in : after(INFINITY);
+            cs.sub = kp.walk_links;
+            probe_t = target;
+            more = target >= t;
+          }
+          // a tiled step is a coarse skip of more than 0.5 (empty_lo_t is at
+          // most that) or evaluates the object: the brute field bounds the
+          // ray's samples from below, the tiled one gives their value
+          const bool brute = OBJ == OBJ_SINGLE_EMPTY || cs.vox_listed == 1u;
+          const uint8_t* field = brute ? kp.brute_field : s.empty_dist;
+          if (!(box_t < 0.0f)) {
+            more = more && walk_start(o, s, field, brute, r, t, end, out);
+            if (!more) end = -1.0f;
+          }
+          uint32_t links = min(cs.sub, kWalkLinks);
+          cs.sub -= links;
 #pragma unroll 1
-    for (uint32_t k = 0; k < kp.interval; ++k) {
-      bool full = true;  // take a full step (index lookups) this iteration
-      // the launch's tail: no work is left to fetch and few lanes march, so
-      // the warp takes their plain clean EMPTY runs together (after the
-      // per-lane block below, where every lane meets again)
-      const bool share = SHARE && exhausted && kp.tail_share && !kp.run_probe &&
-                         static_cast<uint32_t>(__popc(__ballot_sync(kFull, state == ST_MARCH || state == ST_SHADOW))) <=
-                             kp.tail_share;
-      bool pend = false;
-      float pend_lim = 0.0f, pend_dx = 0.0f, pend_dy = 0.0f, pend_dz = 0.0f;
-      uint32_t pend_n = 0;
-      // (a tiled step evaluates the ray's object list only: EMPTY runs need
-      // the voxelized object in it)
-      if (EMPTY_PATH && (state == ST_MARCH || state == ST_SHADOW) && (!MULTI_EMPTY || (cs.vox_listed & 0xFFu))) {
-        // empty-space run: inside a cube of EMPTY blocks every sample is
-        // empty_value(), so up to kp.budget steps run without the sampler.
-        // Several objects: a probe picks the first voxelized object of the
-        // path whose EMPTY cube holds the ray; its constants and balls apply.
-        const bool sh = state == ST_SHADOW;
-        const float dx = sh ? rdx : qdx, dy = sh ? rdy : qdy, dz = sh ? rdz : qdz;
-        const uint32_t max_step = sh ? 256u : p.hard_max_steps;
-        const uint32_t max_near = sh ? 32u : p.scene.max_steps;
-        // a sample below brk goes to the full step, which decides it
-        const float brk = sh ? 0.02f : fmaxf(hit_thr, 0.0f);
-        const float near_thr = sh ? -1.0f : p.near_surface_threshold;
-        const float min_step = sh ? 0.005f : p.min_step;
-        // a ray that may be inside a ball takes full steps until it may have left
-        const bool probe = t > box_t && prev_dist >= kp.probe_min && (!MULTI_EMPTY || t > far_recheck);
-        if (MULTI_EMPTY && probe) {
-          // the set of voxelized objects of the path (that the ray may take
-          // runs on) whose EMPTY cubes hold the ray; the run lasts while it is
-          // in all of them
+          for (; more && links && end < probe_t; --links) more = walk_link(o, s, field, brute, r, end, out);
+          if (more && end < probe_t && cs.sub) {
+            outcome = 0;
+            box_t = -end;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) cs.g[a] = out[a];
+          } else {
+            outcome = more && end >= probe_t ? cs.vox_listed : 0u;
+            if (OBJ == OBJ_SINGLE_EMPTY_TILED && !outcome && cs.vox_listed == 1u) {
+              // not settled: the tiled field's walk, for a run (this phase
+              // again, with no settling ahead)
+              cs.vox_listed = 3u;
+              end = -1.0f;
+              if (cs.hi >= t) end = walk_empty(o, s, s.empty_dist, false, r, t, cs.hi, kp.walk_links);
+            }
+            box_t = end >= t && cs.hi >= t ? fminf(end, cs.hi) : kNoBox;
+            probe_t = cs.lo;
+            // a walk that brought no run of some length puts the next one off
+            const float from = box_t == box_t ? box_t : t;
+            if (probe_t == probe_t && from - t < kShortRun * kp.empty_hi)
+              probe_t = fmaxf(probe_t, from + kPutOff * kp.empty_hi);
+          }
+        } else {
+          box_t = kNoBox;
+          probe_t = after(t);
+          const uint32_t all = (1u << kp.n_ev) - 1u;
+          // ---- how far every object off the path keeps its distance: the first
+          // entry into the ball (box, half-space) of one ahead.  It stays valid
+          // until the ray passes it: balls ahead stay ahead, balls behind stay
+          // behind.  A ray that may be inside one takes full steps until it may
+          // have left.
+          float far_all = cs.g[0];
+          if (t > far_all) {
+            float again;
+            far_all = far_limit(kp.ball, kp.n_ball, all, ox, oy, oz, dx, dy, dz, tmax, t, 0.0f, again);
+            cs.g[0] = far_all < 0.0f ? -1.0f : far_all;
+            if (far_all < 0.0f && again > t) probe_t = again;
+          }
+          // ---- settle: no object below its EMPTY value or ball bound ahead.  Under
+          // the tiled strategy running out of steps needs the exact EMPTY value
+          // of an object every step evaluates.
+          const bool past = t_lo > tmax;
+          const bool masked = MULTI_TILED && !past;
+          const float target = past ? tmax : t_hi;
+          bool exact = past, ok = can && t >= cs.gpos && far_all >= target &&
+                                  (past || (t_hi <= tmax && (!MULTI_TILED || (cs.vox_listed & 0xFFu) == all)));
+          const bool tried = ok;
+          // ---- run: the set of voxelized objects of the path (that the ray may
+          // take runs on) whose EMPTY boxes hold the ray; the run lasts while it
+          // is in all of them
           uint32_t set = 0;
-          box_t = kMaxFloat;
-          for (uint32_t e = 0; e < kp.n_ev; ++e) {
-            if (!((cs.vox_listed >> e) & 1u)) continue;
-            const float bt = probe_empty(sh_objs[kp.ev[e].obj], s.empty_dist, ox, oy, oz, dx, dy, dz, t);
+          float b = kMaxFloat, walk_at = cs.gpos > t ? cs.gpos : after(INFINITY);  // when to walk again
+          for (uint32_t e = 0; e < kp.n_ev && far_all >= 0.0f; ++e) {
+            const bool listed = (cs.vox_listed >> e) & 1u;
+            if (!listed && !ok) continue;
+            const ObjDev& o = sh_objs[kp.ev[e].obj];
+            const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
+            float t_in, t_out;
+            const bool core = core_interval(o, r, t, t_in, t_out);
+            if (listed && core) walk_at = after(t);
+            else if (listed && t_in < t_out && t < t_out) walk_at = fminf(walk_at, fmaxf(t_in, after(t)));
+            float end = -1.0f;
+            // (the tiled strategy's runs need its own field)
+            for (uint32_t pass = ok ? 0u : 1u; pass < 2u; ++pass) {
+              const bool own = pass || masked;
+              if (pass && !(listed && core)) break;
+              end = walk_empty(o, s, own ? s.empty_dist : kp.brute_field, !MULTI_TILED || !own, r, t,
+                               pass ? t_out : target, kp.walk_links);
+              if (!pass) {
+                ok = end >= target;
+                exact = exact || (core && t_out >= target);
+                if (!ok) cs.gpos = fmaxf(end, after(t));
+                if (!MULTI_TILED || ok) break;  // (the brute strategy runs on the same field)
+              }
+            }
+            const float bt = listed && core ? fminf(t_out, end) : -1.0f;
             if (t <= bt) {
               set |= 1u << e;
-              box_t = fminf(box_t, bt);
+              b = fminf(b, bt);
             }
           }
-          if (!set) box_t = -1.0f;
-          if (set && set != (cs.vox_listed >> 8)) {
-            // other objects in the set: the balls that bound the run are others
-            cs.vox_listed = (cs.vox_listed & 0xFFu) | (set << 8);
-            far_t = far_recheck = -1.0f;
-          }
-        }
-        const uint32_t set = MULTI_EMPTY ? (cs.vox_listed >> 8) : 1u;
-        const bool one = (set & (set - 1u)) == 0u;  // one object's EMPTY value
-        const EmptyVox& ev = kp.ev[MULTI_EMPTY ? (__ffs(set | 1u) - 1) : 0];
-        const ObjDev& o0 = sh_objs[MULTI_EMPTY ? ev.obj : 0u];
-        float e_lo = MULTI_EMPTY ? ev.empty_lo : kp.empty_lo;
-        float e_hi = MULTI_EMPTY ? ev.empty_hi : kp.empty_hi;
-        float e_lo_t = MULTI_EMPTY ? ev.empty_lo_t : kp.empty_lo_t;
-        if (MULTI_EMPTY && !one) {
-          for (uint32_t e = 0; e < kp.n_ev; ++e) {
-            if (!((set >> e) & 1u)) continue;
-            e_lo = fminf(e_lo, kp.ev[e].empty_lo);
-            e_lo_t = fminf(e_lo_t, kp.ev[e].empty_lo_t);
-            e_hi = fmaxf(e_hi, kp.ev[e].empty_hi);
-          }
-        }
-        const uint32_t plain = MULTI_EMPTY ? (one ? ev.plain : 0u) : kp.plain_obj;
-        const bool clean = e_lo >= brk && e_lo >= near_thr && e_lo >= min_step;
-        if (probe) {
-          if (!MULTI_EMPTY) box_t = probe_empty(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, t);
-          const float cube_t = box_t;
-          if (MULTI_EMPTY) {
-            // only positions outside the balls of every object not in the set
-            // sample the set's EMPTY values.  far_t (the first entry into such
-            // a ball ahead) stays valid until the ray passes it: balls ahead
-            // stay ahead, balls behind stay behind.
-            if (t <= box_t && t > far_t)
-              far_t = far_limit(kp.ball, kp.n_ball, set, ox, oy, oz, dx, dy, dz, tmax, t, far_recheck);
-            box_t = fminf(box_t, far_t);
-          }
-          if (t <= box_t && clean && one && kp.settle_links && step < max_step && near < max_near) {
-            // Settle the ray if every sample it has left is the EMPTY value:
-            // then no threshold acts on it, it misses, and its outputs do not
-            // depend on its exact t.  t after k more steps lies in
-            // [t + k*lo, t + k*hi] widened by one rounding (2^-24) per step;
-            // 2^-22 per step (and 4 more) leaves room for this bound's own
-            // rounding.  The last sample is the (max_step-step-1)th ahead; the
-            // ray runs out of steps if even its largest t stays <= tmax, and
-            // ends past tmax (with no step flag) if even its smallest t exceeds
-            // tmax.  Either way, when EMPTY cubes cover every position up to
-            // that bound (or tmax), the outcome is settled.
-            const float k = static_cast<float>(max_step - step - 1);
-            const float grow = (k + 4.0f) * 2.384185791015625e-7f;
-            const float t_hi = (t + k * e_hi) * (1.0f + grow);
-            const float t_lo = (t + k * e_lo_t) * (1.0f - grow);
-            const bool out_of_steps = t_hi <= tmax;
-            if (out_of_steps || t_lo > tmax) {
-              const float need = out_of_steps ? t_hi : tmax;
-              if (!MULTI_EMPTY) {
-                box_t = extend_cover(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, box_t, need, kp.settle_links);
-              } else if (far_t >= need) {
-                box_t = fminf(extend_cover(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, cube_t, need, kp.settle_links),
-                              far_t);
+          if (tried && ok && exact) {
+            outcome = past ? 1u : 2u;
+          } else if (far_all >= 0.0f) {
+            if (!(walk_at > after(t)) && walk_at == walk_at) walk_at = after(t);
+            probe_t = walk_at;
+            if (set) {
+              if (set != (cs.vox_listed >> 8)) {
+                // other objects in the set: the balls that bound the run are others
+                cs.vox_listed = (cs.vox_listed & 0xFFu) | (set << 8);
+                far_t = -1.0f;
               }
-              if (box_t >= need) {
-                if (sh) cs.shadow = clampf(cs.shadow, 0.0f, 1.0f);
-                else if (out_of_steps) step = max_step;
-                cs.hit = false;
-                state = ST_EPI;
+              // only positions outside the balls of every object not in the
+              // set sample the set's EMPTY values
+              if (set == all) {
+                far_t = far_all;
+              } else if (t > far_t) {
+                float again;
+                far_t = far_limit(kp.ball, kp.n_ball, set, ox, oy, oz, dx, dy, dz, tmax, t, 0.0f, again);
+                if (far_t < 0.0f && again > t) probe_t = again;
               }
+              box_t = far_t >= t ? fminf(b, far_t) : kNoBox;
             }
+            // a walk that brought no run of some length puts the next one off
+            const float from = box_t == box_t ? box_t : t;
+            const float back = from - t >= 8.0f * kp.empty_hi ? 2.0f * kp.empty_hi
+                                                              : fminf(2.0f * cs.g[1], 16.0f * kp.empty_hi);
+            cs.g[1] = back;
+            if (probe_t == probe_t) probe_t = fmaxf(probe_t, from + back);
           }
         }
-        if (state != ST_EPI && t <= box_t) {
-          const uint32_t n = step < max_step ? min(kp.budget, max_step - step) : 0u;
-          uint32_t c = 0;
-          bool stop_full = true;
-          if (near < max_near && MULTI_EMPTY && !one) {
-            // several objects: the least of their EMPTY values, to the end of
-            // the nearest cube
-            c = clean ? empty_run_set<true>(sh_objs, kp.ev, set, kp.n_ev, ox, oy, oz, dx, dy, dz, tmax, n, brk,
-                                            near_thr, min_step, max_near, t, box_t, prev_t, prev_dist, near, stop_full)
-                      : empty_run_set<false>(sh_objs, kp.ev, set, kp.n_ev, ox, oy, oz, dx, dy, dz, tmax, n, brk,
-                                             near_thr, min_step, max_near, t, box_t, prev_t, prev_dist, near,
-                                             stop_full);
-          } else if (near < max_near) {
-#define RKF_RUN(P, CL, IN)                                                                                   \
-  empty_run<P, CL, IN, MULTI_EMPTY>(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, tmax, n, brk, near_thr, min_step, \
-                                    max_near, far_t, t, box_t, prev_t, prev_dist, near, stop_full)
-            if (plain && clean && share) {
-              // the whole run at once (the budget only paces warps that share
-              // nothing); taken with the warp below
-              pend = true;
-              pend_lim = fminf(box_t, tmax);
-              pend_n = step < max_step ? max_step - step : 0u;
-              pend_dx = dx;
-              pend_dy = dy;
-              pend_dz = dz;
-            } else if (plain && clean)
-              c = kp.run_probe ? empty_run_x2<true, MULTI_EMPTY>(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, tmax, n,
-                                                                 far_t, t, box_t, prev_t, prev_dist, stop_full)
-                               : empty_run_x2<false, MULTI_EMPTY>(o0, s.empty_dist, ox, oy, oz, dx, dy, dz, tmax, n,
-                                                                  far_t, t, box_t, prev_t, prev_dist, stop_full);
-            else if (plain)
-              c = kp.run_probe ? RKF_RUN(true, false, true) : RKF_RUN(true, false, false);
-            else
-              c = kp.run_probe ? RKF_RUN(false, false, true) : RKF_RUN(false, false, false);
-#undef RKF_RUN
-          }
-          step += c;
-          // a run that used its whole budget, or reached the end of its cube
-          // between probes, continues next iteration unless a limit ends the
-          // ray; any other stop needs the full step's decision
-          full = stop_full || step >= max_step || t > tmax || near >= max_near;
-        }
-      }
-      if (share) {  // warp-uniform: every lane is here
-        uint32_t c = 0;
-        bool stop_full = false;
-        shared_runs(sh_objs[0], pend, ox, oy, oz, pend_dx, pend_dy, pend_dz, pend_lim, tmax, pend_n, t, prev_t,
-                    prev_dist, c, stop_full);
-        if (pend) {
-          const bool sh = state == ST_SHADOW;
-          step += c;
-          full = stop_full || step >= (sh ? 256u : p.hard_max_steps) || t > tmax ||
-                 near >= (sh ? 32u : p.scene.max_steps);
-        }
-      }
-      if (!full) {
-      } else if (state == ST_MARCH) {
-        if (step >= p.hard_max_steps || t > tmax || near >= p.scene.max_steps) {
-          cs.hit = false;
+        if (outcome) {
+          if (!sh && outcome == 2) step = max_step;
           state = ST_EPI;
-        } else {
-          float best_un;
-          uint32_t best_i;
-          const float wx = __fadd_rn(ox, __fmul_rn(qdx, t)), wy = __fadd_rn(oy, __fmul_rn(qdy, t)),
-                      wz = __fadd_rn(oz, __fmul_rn(qdz, t));
-          float best;
-          bool skipped = false;
-          if (TILES && kp.tiled && cs.tile_count != kNoTiles) {
-            // ray_march_tiled (:899-938): a coarse empty-space skip, else the
-            // tile's objects only
-            const Segment& sg = kp.segs[cs.seg];
-            const float cd = coarse_sample(kp.td, sg.coarse_ocr, __fsub_rn(wx, sg.pos[0]), __fsub_rn(wy, sg.pos[1]),
-                                           __fsub_rn(wz, sg.pos[2]));
-            best = kMaxFloat;
-            best_un = kMaxFloat;
-            best_i = 0;
-            if (cd > kCoarseNear) {
-              prev_dist = kMaxFloat;
-              t = __fadd_rn(t, cd);
-              step++;
-              skipped = true;
-            } else {
-              for (uint32_t j = 0; j < cs.tile_count; ++j) {
-                const uint32_t oi = __ldg(kp.td.tile_list + cs.tile_base + j);
-                float du;
-                const float d = eval_obj<PREC>(s, sh_objs[oi], wx, wy, wz, &du, lc);
-                if (d < best) {
-                  best = d;
-                  best_un = du;
-                  best_i = oi;
-                }
-              }
-            }
-          } else if ((!EMPTY_PATH || MULTI_EMPTY) && kp.use_bvh) {
-            best = eval_bvh<PREC>(s, sh_objs, kp.bvh, kp.bvh_next, nobj, wx, wy, wz, best_un, best_i, lc);
-          } else {
-            best = eval_min<PREC, SINGLE>(s, sh_objs, 0, nobj, wx, wy, wz, best_un, best_i, lc);
-          }
-          if (skipped) {
-          } else if (best < 0.0f && prev_dist > hit_thr) {  // overstep (ray_march.wgsl:816)
-            cs.hit_obj = best_i;
-            cs.hit = true;
-            if (mode == RKF_TRACE_ANY) {
-              state = ST_EPI;
-            } else {
-              cs.lo = prev_t;
-              cs.hi = t;
-              cs.mat_t = t;
-              cs.mat_ok = best_un < sh_objs[best_i].vs16;
-              cs.sub = 0;
-              cs.bisected = true;
-              state = ST_BISECT;
-            }
-          } else if (best < hit_thr) {  // :842
-            cs.hit_obj = best_i;
-            cs.hit = true;
-            if (mode == RKF_TRACE_ANY) {
-              state = ST_EPI;
-            } else {
-              // a direct cs.hit: enter the finish phase with the bisection done
-              cs.mat_t = t;
-              cs.mat_ok = best_un < sh_objs[best_i].vs16;
-              cs.sub = p.bisect_steps;
-              state = ST_BISECT;
-            }
-          } else {
-            if (best < p.near_surface_threshold) near++;
-            prev_t = t;
-            prev_dist = best;
-            t = __fadd_rn(t, fmax_(best, p.min_step));
-            step++;
-          }
-        }
-      } else if (state == ST_SHADOW) {
-        // soft_shadow (shade_common_shading.wgsl:9-33)
-        if (step >= 256u || near >= 32u || t > tmax) {
-          cs.shadow = clampf(cs.shadow, 0.0f, 1.0f);
-          cs.hit = false;
-          state = ST_EPI;
-        } else {
-          float best_un;
-          uint32_t best_i;
-          const float best = eval_min<PREC, SINGLE>(s, sh_objs, 0, nobj, __fadd_rn(ox, __fmul_rn(rdx, t)),
-                                                    __fadd_rn(oy, __fmul_rn(rdy, t)),
-                                                    __fadd_rn(oz, __fmul_rn(rdz, t)), best_un, best_i, lc);
-          prev_dist = best;
-          if (best < 0.005f) {
-            cs.shadow = 0.0f;
-            cs.hit = true;
-            state = ST_EPI;
-          } else {
-            if (best < 0.02f) {
-              cs.shadow = fmin_(cs.shadow, __fdiv_rn(__fmul_rn(16.0f, best), t));
-              near++;
-            }
-            t = __fadd_rn(t, fmax_(best, 0.005f));
-            step++;
-          }
         }
       }
-      // leave to finish and refill once refill_idle lanes are done (or,
-      // with no work left to fetch, once none is marching)
-      const uint32_t active = __popc(__ballot_sync(kFull, state == ST_MARCH || state == ST_SHADOW));
-      if (active <= (exhausted ? 0u : kp.refill_active)) break;
+      continue;
     }
 
-    // ---- 3. finish: bisection and central differences -------------------------
-    float g0 = 0, g1 = 0, g2 = 0, lpx = 0, lpy = 0, lpz = 0, eps = 0;
-    while (__any_sync(kFull, state == ST_BISECT || state == ST_NORMAL)) {
-      if (state == ST_BISECT && cs.sub >= p.bisect_steps) {
-        // bisection done (or a direct cs.hit): t = (cs.lo+cs.hi)/2, set up the normal
-        if (cs.bisected) t = __fmul_rn(__fadd_rn(cs.lo, cs.hi), 0.5f);
-        const ObjDev& o = sh_objs[cs.hit_obj];
-        const float hx = __fadd_rn(ox, __fmul_rn(rdx, t));
-        const float hy = __fadd_rn(oy, __fmul_rn(rdy, t));
-        const float hz = __fadd_rn(oz, __fmul_rn(rdz, t));
-        if (o.sdf_type == RKF_SDF_VOXELIZED) {
-          to_local_fast(o, hx, hy, hz, lpx, lpy, lpz);
-          eps = __fmul_rn(o.vs, 2.0f);
+    if (EMPTY_PATH && n_run && n_run >= n_eval) {
+      // ---- run: up to kp.budget steps over EMPTY samples, without the sampler ------
+      if (run) {
+        // several objects: the set's EMPTY values (of one object, its constants)
+        const uint32_t set = MULTI_EMPTY ? (cs.vox_listed >> 8) : 1u;
+        const bool one = (set & (set - 1u)) == 0u;
+        const EmptyVox& ev = kp.ev[MULTI_EMPTY ? (__ffs(set | 1u) - 1) : 0];
+        const ObjDev& o0 = sh_objs[MULTI_EMPTY ? ev.obj : 0u];
+        const uint32_t plain = MULTI_EMPTY ? (one ? ev.plain : 0u) : kp.plain_obj;
+        // (the path's least lower bound: no set's is below it)
+        const bool clean = kp.empty_lo >= brk && kp.empty_lo >= near_thr && kp.empty_lo >= min_step;
+        const uint32_t n = min(kp.budget, max_step - step);
+        uint32_t c = 0;
+        bool stop_full = true;
+        if (MULTI_EMPTY && !one) {
+          // several objects: the least of their EMPTY values, to the end of
+          // the nearest cube
+          c = clean ? empty_run_set<true>(sh_objs, kp.ev, set, kp.n_ev, ox, oy, oz, dx, dy, dz, tmax, n, brk,
+                                          near_thr, min_step, max_near, t, box_t, prev_t, prev_dist, near, stop_full)
+                    : empty_run_set<false>(sh_objs, kp.ev, set, kp.n_ev, ox, oy, oz, dx, dy, dz, tmax, n, brk,
+                                           near_thr, min_step, max_near, t, box_t, prev_t, prev_dist, near,
+                                           stop_full);
+        } else if (plain && clean) {
+          c = empty_run_x2(o0, ox, oy, oz, dx, dy, dz, tmax, n, t, box_t, prev_t, prev_dist, stop_full);
+        } else if (plain) {
+          c = empty_run<true>(o0, ox, oy, oz, dx, dy, dz, tmax, n, brk, near_thr, min_step, max_near, t, box_t,
+                              prev_t, prev_dist, near, stop_full);
         } else {
-          lpx = hx;
-          lpy = hy;
-          lpz = hz;
-          eps = __fmul_rn(hit_thr, 10.0f);
+          c = empty_run<false>(o0, ox, oy, oz, dx, dy, dz, tmax, n, brk, near_thr, min_step, max_near, t, box_t,
+                               prev_t, prev_dist, near, stop_full);
         }
+        step += c;
+        if (step >= max_step || t > tmax || near >= max_near) {
+          state = ST_EPI;
+        } else if (stop_full || t > box_t) {
+          // past the covered interval (or at a sample a threshold acts on)
+          // comes an evaluated step
+          box_t = kNoBox;
+          probe_t = after(t);
+        }
+      }
+      continue;
+    }
+
+    // ---- eval: a sample of each lane that needs one, and on while most do --------
+    bool eval = !done && !walk && !run;
+#pragma unroll 1
+    for (uint32_t rep = 0; rep < kEvalReps; ++rep) {
+    if (eval) {
+      if (state == ST_BISECT && cs.sub >= p.bisect_steps) {
+        // bisection done (or a direct hit): t = (lo+hi)/2, on to the normal
+        if (cs.bisected) t = __fmul_rn(__fadd_rn(cs.lo, cs.hi), 0.5f);
         cs.sub = 0;
         state = ST_NORMAL;
       }
-      if (state == ST_BISECT) {
+      float best = kMaxFloat, best_un = kMaxFloat;
+      uint32_t best_i = 0;
+      bool skipped = false;
+      float px, py, pz;       // the position: world space, or object-local for a voxelized object's normal
+      bool local = false;     // px..pz are object-local
+      bool grad = false;      // the gradient's sampler
+      bool only = false;      // the hit object alone, whatever its value
+      uint32_t jb = 0, je = SINGLE ? 1u : nobj;
+      if (state == ST_NORMAL) {
+        px = __fadd_rn(ox, __fmul_rn(rdx, t));
+        py = __fadd_rn(oy, __fmul_rn(rdy, t));
+        pz = __fadd_rn(oz, __fmul_rn(rdz, t));
+        const ObjDev& o = sh_objs[SINGLE ? 0u : cs.hit_obj];
+        float eps = __fmul_rn(hit_thr, 10.0f);
+        if (PLAIN_VOX || o.sdf_type == RKF_SDF_VOXELIZED) {
+          to_local_fast(o, px, py, pz, px, py, pz);
+          eps = __fmul_rn(o.vs, 2.0f);
+          local = true;
+          grad = cs.sub < 6u;  // the 7th sample: the hit's own distance (motion plane)
+        }
+        const uint32_t ax = cs.sub >> 1;
+        if (cs.sub & 1u) eps = -eps;  // x + (-eps) is x - eps
+        if (ax == 0) px = __fadd_rn(px, eps);
+        if (ax == 1) py = __fadd_rn(py, eps);
+        if (ax == 2) pz = __fadd_rn(pz, eps);
+        only = true;
+      } else {
+        const float ts = state == ST_BISECT ? __fmul_rn(__fadd_rn(cs.lo, cs.hi), 0.5f) : t;
+        px = __fadd_rn(ox, __fmul_rn(dx, ts));
+        py = __fadd_rn(oy, __fmul_rn(dy, ts));
+        pz = __fadd_rn(oz, __fmul_rn(dz, ts));
+        only = state == ST_BISECT;
+      }
+      bool list = false;
+      if (!SINGLE && only) {
+        jb = cs.hit_obj;
+        je = jb + 1u;
+      }
+      if (TILES && kp.tiled && state == ST_MARCH && cs.tile_count != kNoTiles) {
+        // ray_march_tiled (:899-938): a coarse empty-space skip, else the
+        // tile's objects only
+        const Segment& sg = kp.segs[cs.seg];
+        const float cd = coarse_sample(kp.td, sg.coarse_ocr, __fsub_rn(px, sg.pos[0]), __fsub_rn(py, sg.pos[1]),
+                                       __fsub_rn(pz, sg.pos[2]));
+        if (cd > kCoarseNear) {
+          prev_dist = kMaxFloat;
+          t = __fadd_rn(t, cd);
+          step++;
+          skipped = true;
+          je = 0;
+        } else {
+          list = true;
+          je = cs.tile_count;
+        }
+      }
+      if ((!EMPTY_PATH || OBJ == OBJ_MULTI_EMPTY) && kp.use_bvh && state == ST_MARCH) {
+        best = eval_bvh<PREC>(s, sh_objs, kp.bvh, kp.bvh_next, nobj, px, py, pz, best_un, best_i);
+        je = 0;
+      }
+      for (uint32_t j = jb; j < je; ++j) {
+        const uint32_t oi = list ? __ldg(kp.td.tile_list + cs.tile_base + j) : j;
+        const ObjDev& o = sh_objs[SINGLE ? 0u : oi];
+        float d = kMaxFloat, du = kMaxFloat;
+        if (PLAIN_VOX) {  // one voxelized object, translation only
+          const float lx = local ? px : __fadd_rn(px, o.m[12]), ly = local ? py : __fadd_rn(py, o.m[13]),
+                      lz = local ? pz : __fadd_rn(pz, o.m[14]);
+          du = sample_vox<PREC, true>(s, o, lx, ly, lz, grad, lc);
+          d = local ? du : __fmul_rn(du, o.min_scale);
+        } else if (o.sdf_type != RKF_SDF_NONE) {
+          float lx = px, ly = py, lz = pz;
+          if (!local) to_local_fast(o, px, py, pz, lx, ly, lz);
+          du = o.sdf_type == RKF_SDF_ANALYTICAL ? analytic_sdf(o, lx, ly, lz)
+                                                : sample_vox<PREC>(s, o, lx, ly, lz, grad, lc);
+          d = local ? du : __fmul_rn(du, o.min_scale);
+        }
+        if ((SINGLE && !list) || only || d < best) {
+          best = d;
+          best_un = du;
+          best_i = oi;
+        }
+      }
+      // ---- what the sample decides ------------------------------------------------
+      if (state == ST_MARCH) {
+        if (skipped) {
+        } else if (best < 0.0f && prev_dist > hit_thr) {  // overstep (ray_march.wgsl:816)
+          cs.hit_obj = best_i;
+          cs.hit = true;
+          cs.lo = prev_t;
+          cs.hi = t;
+          cs.mat_t = t;
+          cs.mat_ok = best_un < sh_objs[best_i].vs16;
+          cs.sub = 0;
+          cs.bisected = true;
+          state = mode == RKF_TRACE_ANY ? ST_EPI : ST_BISECT;
+        } else if (best < hit_thr) {  // :842
+          // a direct hit: the bisection is done
+          cs.hit_obj = best_i;
+          cs.hit = true;
+          cs.mat_t = t;
+          cs.mat_ok = best_un < sh_objs[best_i].vs16;
+          cs.sub = p.bisect_steps;
+          state = mode == RKF_TRACE_ANY ? ST_EPI : ST_BISECT;
+        } else {
+          if (best < p.near_surface_threshold) near++;
+          prev_t = t;
+          prev_dist = best;
+          t = __fadd_rn(t, fmax_(best, p.min_step));
+          step++;
+        }
+        if (state == ST_MARCH && (step >= p.hard_max_steps || t > tmax || near >= p.scene.max_steps)) state = ST_EPI;
+      } else if (state == ST_SHADOW) {
+        // soft_shadow (shade_common_shading.wgsl:9-33)
+        prev_dist = best;
+        if (best < 0.005f) {
+          cs.shadow = 0.0f;
+          cs.hit = true;
+          state = ST_EPI;
+        } else {
+          if (best < 0.02f) {
+            cs.shadow = fmin_(cs.shadow, __fdiv_rn(__fmul_rn(16.0f, best), t));
+            near++;
+          }
+          t = __fadd_rn(t, fmax_(best, 0.005f));
+          step++;
+          if (step >= 256u || near >= 32u || t > tmax) state = ST_EPI;
+        }
+      } else if (state == ST_BISECT) {
         const float mid = __fmul_rn(__fadd_rn(cs.lo, cs.hi), 0.5f);
-        float du;
-        const float d = eval_obj<PREC>(s, sh_objs[cs.hit_obj], __fadd_rn(ox, __fmul_rn(qdx, mid)),
-                                       __fadd_rn(oy, __fmul_rn(qdy, mid)), __fadd_rn(oz, __fmul_rn(qdz, mid)),
-                                       &du, lc);
-        if (d < 0.0f) {
+        if (best < 0.0f) {
           cs.hi = mid;
         } else {
           cs.lo = mid;
           cs.mat_t = mid;
-          cs.mat_ok = du < sh_objs[cs.hit_obj].vs16;
+          cs.mat_ok = best_un < sh_objs[SINGLE ? 0u : cs.hit_obj].vs16;
         }
         ++cs.sub;
-      } else if (state == ST_NORMAL) {
-        const ObjDev& o = sh_objs[cs.hit_obj];
-        const uint32_t ax = cs.sub >> 1;
-        float qx = lpx, qy = lpy, qz = lpz;
-        if (ax == 0) qx = (cs.sub & 1) ? __fsub_rn(lpx, eps) : __fadd_rn(lpx, eps);
-        if (ax == 1) qy = (cs.sub & 1) ? __fsub_rn(lpy, eps) : __fadd_rn(lpy, eps);
-        if (ax == 2) qz = (cs.sub & 1) ? __fsub_rn(lpz, eps) : __fadd_rn(lpz, eps);
-        float d;
-        if (o.sdf_type == RKF_SDF_VOXELIZED) {
-          d = sample_vox<PREC>(s, o, qx, qy, qz, true, lc);
+      } else {  // ST_NORMAL
+        const uint32_t sub = cs.sub;
+        if (sub >= 6u) {
+          cs.sdf_hit = best;
+          state = ST_EPI;
+        } else if (sub & 1u) {
+          cs.g[sub >> 1] = __fsub_rn(cs.gpos, best);
+          if (sub == 5u && !(local && kp.segs[cs.seg].motion)) state = ST_EPI;
         } else {
-          float du;
-          d = eval_obj<PREC>(s, o, qx, qy, qz, &du, lc);
+          cs.gpos = best;
         }
-        if (cs.sub & 1) {
-          const float g = __fsub_rn(cs.gpos, d);
-          if (ax == 0) g0 = g;
-          else if (ax == 1) g1 = g;
-          else g2 = g;
-        } else {
-          cs.gpos = d;
-        }
-        if (++cs.sub == 6) state = ST_EPI;
+        cs.sub = sub + 1u;
       }
+      eval = state == ST_BISECT || state == ST_NORMAL ||
+             ((state == ST_MARCH || state == ST_SHADOW) &&
+              !(EMPTY_PATH && t >= probe_t && prev_dist >= kp.probe_min));
     }
-
-    // ---- 4. epilogue: outputs of finished rays -------------------------------
-    if (state == ST_EPI) {
-      const Segment& sg = kp.segs[cs.seg];
-      if (mode == RKF_TRACE_SHADOW) {
-        sg.t[cs.idx] = cs.shadow;
-        if (sg.flags) sg.flags[cs.idx] = cs.hit ? RKF_FLAG_HIT : 0;
-      } else if (mode == RKF_TRACE_ANY) {
-        sg.t[cs.idx] = cs.hit ? t : kMaxFloat;
-        if (sg.flags)
-          sg.flags[cs.idx] = cs.hit ? RKF_FLAG_HIT
-                              : ((step >= p.hard_max_steps || near >= p.scene.max_steps) ? RKF_FLAG_STEPS_OUT : 0);
-      } else {
-        uint16_t flags = 0;
-        float nx = 0, ny = 0, nz = 0;
-        uint32_t slot = RKF_EMPTY_SLOT, mat = 0, sec = 0, blend = 0;
-        float hx = 0, hy = 0, hz = 0, sdf_hit = 0;
-        if (cs.hit) {
-          flags |= RKF_FLAG_HIT;
-          if (cs.bisected) flags |= RKF_FLAG_BISECTED;
-          const ObjDev& o = sh_objs[cs.hit_obj];
-          hx = __fadd_rn(ox, __fmul_rn(rdx, t));
-          hy = __fadd_rn(oy, __fmul_rn(rdy, t));
-          hz = __fadd_rn(oz, __fmul_rn(rdz, t));
-          if (o.sdf_type == RKF_SDF_VOXELIZED) {
-            // world_grad = transpose(inverse_world) * (g, 0)  (:1014)
-            const float wx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[0], g0), __fmul_rn(o.m[1], g1)),
-                                                 __fmul_rn(o.m[2], g2)), __fmul_rn(o.m[3], 0.0f));
-            const float wy = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[4], g0), __fmul_rn(o.m[5], g1)),
-                                                 __fmul_rn(o.m[6], g2)), __fmul_rn(o.m[7], 0.0f));
-            const float wz = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[8], g0), __fmul_rn(o.m[9], g1)),
-                                                 __fmul_rn(o.m[10], g2)), __fmul_rn(o.m[11], 0.0f));
-            const float l = len3(wx, wy, wz);
-            if (l < 1e-10f) {
-              ny = 1.0f;
-            } else {
-              nx = __fdiv_rn(wx, l); ny = __fdiv_rn(wy, l); nz = __fdiv_rn(wz, l);
-            }
-            uint32_t vi = 0;
-            slot = nearest_slot(s, o, lpx, lpy, lpz, vi, lc);
-            if (slot < RKF_INTERIOR_SLOT) {
-              const size_t v = static_cast<size_t>(slot) * 512 + vi;
-              sec = (__ldg(s.mat + v) >> 6) & 0x3Fu;
-              blend = __ldg(s.blend + v);
-            }
-            if (sg.motion) sdf_hit = sample_vox<PREC>(s, o, lpx, lpy, lpz, false, lc);
-          } else {
-            const float l = len3(g0, g1, g2);
-            nx = __fdiv_rn(g0, l); ny = __fdiv_rn(g1, l); nz = __fdiv_rn(g2, l);
-          }
-          if (cs.mat_ok || o.sdf_type == RKF_SDF_ANALYTICAL)
-            mat = material_at(s, o, __fadd_rn(ox, __fmul_rn(qdx, cs.mat_t)), __fadd_rn(oy, __fmul_rn(qdy, cs.mat_t)),
-                              __fadd_rn(oz, __fmul_rn(qdz, cs.mat_t)), lc);
-        } else if (step >= p.hard_max_steps || near >= p.scene.max_steps) {
-          flags |= RKF_FLAG_STEPS_OUT;
-        }
-        sg.t[cs.idx] = cs.hit ? t : kMaxFloat;
-        if (sg.normal) {
-          sg.normal[3 * static_cast<size_t>(cs.idx)] = nx;
-          sg.normal[3 * static_cast<size_t>(cs.idx) + 1] = ny;
-          sg.normal[3 * static_cast<size_t>(cs.idx) + 2] = nz;
-        }
-        if (sg.slot) sg.slot[cs.idx] = slot;
-        if (sg.material) sg.material[cs.idx] = static_cast<uint16_t>(mat);
-        if (sg.flags) sg.flags[cs.idx] = flags;
-        if (sg.position) {
-          const float4 pv = cs.hit ? make_float4(hx, hy, hz, t) : make_float4(0.f, 0.f, 0.f, kMaxFloat);
-          reinterpret_cast<float4*>(sg.position)[cs.idx] = pv;
-        }
-        if (sg.packed)
-          sg.packed[cs.idx] = cs.hit ? ((mat & 0x3Fu) | (sec << 6) | (blend << 12) | (sh_objs[cs.hit_obj].object_id << 24))
-                               : 0u;
-        if (sg.motion) {
-          float4 mv = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (cs.hit) {
-            const float* m = sg.prev_vp;  // ray_march.wgsl:1094-1105
-            const float cx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[0], hx), __fmul_rn(m[4], hy)),
-                                                 __fmul_rn(m[8], hz)), __fmul_rn(m[12], 1.0f));
-            const float cy = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[1], hx), __fmul_rn(m[5], hy)),
-                                                 __fmul_rn(m[9], hz)), __fmul_rn(m[13], 1.0f));
-            const float cw = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(m[3], hx), __fmul_rn(m[7], hy)),
-                                                 __fmul_rn(m[11], hz)), __fmul_rn(m[15], 1.0f));
-            float mox = 0.f, moy = 0.f;
-            if (cw > 0.0f) {
-              const float ndx = __fdiv_rn(cx, cw), ndy = __fdiv_rn(cy, cw);
-              const float pu = __fadd_rn(__fmul_rn(ndx, 0.5f), 0.5f);
-              const float pv = __fsub_rn(0.5f, __fmul_rn(ndy, 0.5f));
-              const uint32_t px = cs.idx % sg.w, py = cs.idx / sg.w;
-              const float cu = __fdiv_rn(__fadd_rn(static_cast<float>(px), 0.5f), static_cast<float>(sg.w));
-              const float cv = __fdiv_rn(__fadd_rn(static_cast<float>(py), 0.5f), static_cast<float>(sg.h));
-              mox = __fsub_rn(cu, pu);
-              moy = __fsub_rn(cv, pv);
-            }
-            mv = make_float4(mox, moy, 1.0f, sdf_hit);
-          }
-          reinterpret_cast<float4*>(sg.motion)[cs.idx] = mv;
-        }
-      }
-      state = ST_IDLE;
+    if (2 * __popc(__ballot_sync(kFull, eval)) < n_eval) break;
     }
   }
 }
@@ -1780,6 +1479,37 @@ bool fill_multi_empty(const Ctx* c, bool walk, detail::KParams& kp) {
   return kp.n_ev > 0;
 }
 
+// The bounds of the EMPTY values of the launch's path: of object 0, or of the
+// path's objects together (filled by fill_multi_empty).  mix(c, c, t) three
+// times stays within 12 roundings of c (relative 2^-24 each): 0.999 leaves a
+// wide margin, 2^-16 a tight one.  A tiled launch also steps by coarse skips,
+// each of more than kCoarseNear.
+void empty_bounds(detail::KParams& kp, bool empty, bool multi, bool tiled) {
+  const ObjDev& e0 = kp.objs[0];
+  kp.probe_min = empty ? (multi ? kp.probe_min : 0.99f * e0.be * e0.min_scale) : kMaxFloat;
+  kp.empty_lo = empty ? 0.999f * e0.be * e0.min_scale : 0.0f;
+  kp.empty_lo_t = e0.be * e0.min_scale * (1.0f - 1.52587890625e-5f);
+  kp.empty_hi = empty_hi_of(e0);
+  for (uint32_t e = 0; multi && e < kp.n_ev; ++e) {
+    const detail::EmptyVox& v = kp.ev[e];
+    kp.empty_lo = e ? std::min(kp.empty_lo, v.empty_lo) : v.empty_lo;
+    kp.empty_lo_t = e ? std::min(kp.empty_lo_t, v.empty_lo_t) : v.empty_lo_t;
+    kp.empty_hi = e ? std::max(kp.empty_hi, v.empty_hi) : v.empty_hi;
+  }
+  if (tiled) kp.empty_lo_t = std::min(kp.empty_lo_t, kCoarseNear);
+  kp.walk_links = 64;
+}
+
+constexpr float kFewSteps = 150.0f, kFewStepsTiled = 250.0f;
+// Every grid of the path at most `steps` EMPTY steps long.
+bool few_empty_steps(const detail::KParams& kp, bool multi, float steps) {
+  for (uint32_t e = 0; e < (multi ? kp.n_ev : 1u); ++e) {
+    const ObjDev& o = kp.objs[multi ? kp.ev[e].obj : 0u];
+    if (2.0f * std::max({o.half_gs[0], o.half_gs[1], o.half_gs[2]}) > steps * o.be) return false;
+  }
+  return true;
+}
+
 // Which kernel variant a launch over this context's objects uses.
 int object_set(const Ctx* c) {
   if (c->obj_count() != 1)
@@ -1852,7 +1582,14 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   OrderTable order_tbl;
   bool ordered = false;
   std::vector<Segment> ordered_segs;
-  if (tu.order_tiles && id0 == 0 && !segs_resident && !tiled && empty_order_source(c, p, tu, &order_obj)) {
+  // the settling passes take the place of that order: what they leave is an
+  // even list of rays
+  uint64_t view_ids = 0;
+  for (const Segment& sg : segs_host)
+    if (sg.kind == 0) view_ids += sg.n_ids;
+  const bool settle = (objs == detail::OBJ_SINGLE_EMPTY || objs == detail::OBJ_MULTI_EMPTY) && id0 == 0 &&
+                      !segs_resident && view_ids >= kSettleIds && view_ids < (1ull << 32);
+  if (tu.order_tiles && !settle && id0 == 0 && !segs_resident && !tiled && empty_order_source(c, p, tu, &order_obj)) {
     ordered_segs = segs_host;
     rkf_status s2 = tile_order_prepare(c, ordered_segs, tu.tile_w, tu.tile_h, nullptr, 0, &order_tbl, &ordered);
     if (s2 != RKF_OK) return s2;
@@ -1915,19 +1652,38 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   kp.bvh_next = walk ? c->bvh_next.as<uint32_t>() : nullptr;
   kp.use_bvh = walk ? 1u : 0u;
   const ObjDev& e0 = kp.objs[0];  // the object of the single-object empty-space path
-  if (!multi_empty) kp.probe_min = empty ? 0.99f * e0.be * e0.min_scale : kMaxFloat;
+  empty_bounds(kp, empty, multi_empty, tiled);
   kp.budget = tu.step_budget ? tu.step_budget : 32;
-  kp.refill_active = 32u - std::min<uint32_t>(tu.refill_idle ? tu.refill_idle : 32u, 32u);
-  kp.run_probe = tu.probe_in_run ? 1u : 0u;
-  kp.tail_share = std::min<uint32_t>(tu.tail_share, 32u);
-  // mix(c, c, t) three times stays within 12 roundings of c (relative 2^-24
-  // each); 0.999 leaves a wide margin
-  kp.empty_lo = empty ? 0.999f * e0.be * e0.min_scale : 0.0f;
-  // twelve roundings of 2^-24 stay far inside 2^-16
-  kp.empty_lo_t = e0.be * e0.min_scale * (1.0f - 1.52587890625e-5f);
-  kp.empty_hi = empty_hi_of(e0);
-  kp.settle_links = empty ? 48u : 0u;
+  kp.brute_field = c->empty_dist.as<uint8_t>();
   kp.plain_obj = (e0.m[12] == 0.0f && e0.m[13] == 0.0f && e0.m[14] == 0.0f && e0.min_scale == 1.0f) ? 1u : 0u;
+  const uint32_t threads = tu.threads_per_block ? tu.threads_per_block : 256;
+  if (threads > 256 || threads % 32)
+    return fail(RKF_INVALID_ARG, "march: threads_per_block must be a multiple of 32 <= 256");
+  // Several objects whose grids are few EMPTY steps across leave few of them to
+  // a run: after the settling passes the rays that are left march the plain
+  // kernel, whose loop is the shorter one (1277x717, five objects, grids 100
+  // EMPTY steps a side: 1.86 / 1.72 / 2.27 ms against 2.72 / 3.44 / 3.55 under
+  // brute / tiled / BVH; 200 steps: 1.77 / 1.43 / 1.79 against 1.46 / 1.76 /
+  // 1.77; 400 steps: 7.5 / 4.3 / 7.1 against 2.7 / 1.8 / 2.7).  Else the tiled
+  // strategy goes without the passes: its coarse skips leave the misses cheap
+  // (grids of 1,600 steps: 1.75 ms against 2.22 with them).  One object: u8,
+  // 1920x1080, 100 steps: 1.64 ms plain against 2.29; 200 steps: 0.90 either way;
+  // 400 steps: 1.15 against 0.59.  Tiled (plain also without the passes):
+  // 100 steps 1.30 ms against 5.9, 200 steps 1.08 against 1.47, 400 steps 3.1
+  // against 1.0.
+  const bool few = empty && few_empty_steps(kp, multi_empty, tiled ? kFewStepsTiled : kFewSteps);
+  const bool tiled_empty = tiled && empty;
+  if (settle && empty && (!tiled_empty || few)) {
+    const size_t need = settle_bytes(view_ids, kp.tile_w * kp.tile_h);
+    if (c->settle_buf.bytes >= need || c->settle_buf.alloc(need + need / 8) == RKF_OK) {
+      const rkf_status s2 = settle_enqueue(c, kp, obj, view_ids, c->settle_buf.p, st);
+      if (s2 != RKF_OK) return s2;
+      if (few) obj = multi_empty ? detail::OBJ_MULTI : detail::OBJ_SINGLE;
+    } else {
+      cudaGetLastError();  // no room for the lists: the march alone
+    }
+  }
+  if (few && obj == detail::OBJ_SINGLE_EMPTY_TILED) obj = detail::OBJ_SINGLE;
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
@@ -1940,9 +1696,7 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
       fn = detail::persistent_fn<RKF_PRECISION_F16>(obj);
   }
   c->last_variant = obj;
-  const uint32_t threads = tu.threads_per_block ? tu.threads_per_block : 256;
-  if (threads > 256 || threads % 32)
-    return fail(RKF_INVALID_ARG, "march: threads_per_block must be a multiple of 32 <= 256");
+  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj);
   const size_t smem = 0;
   uint32_t bps = tu.blocks_per_sm;
   if (bps == 0) {
@@ -1950,9 +1704,9 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
     RKF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
     bps = occ > 0 ? static_cast<uint32_t>(occ) : 1;
   }
-  // never launch more lanes than work items
   uint64_t blocks = static_cast<uint64_t>(c->sm_count) * bps;
-  const uint64_t need_blocks = (total + threads - 1) / threads;
+  const uint64_t block_rays = threads / 32 * detail::kLeastLanes;  // (lane_share spreads them)
+  const uint64_t need_blocks = (total + block_rays - 1) / block_rays;
   if (blocks > need_blocks) blocks = need_blocks ? need_blocks : 1;
   void* args[] = {&kp};
   rkf_status se = c->march_event(st, false);
@@ -2002,18 +1756,10 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
   const bool memp = obj == detail::OBJ_MULTI_EMPTY;
   const ObjDev& e0 = kp.objs[0];  // the object of the single-object empty-space path
   const bool empty = obj == detail::OBJ_SINGLE_EMPTY || memp;
-  if (!memp) kp.probe_min = empty ? 0.99f * e0.be * e0.min_scale : kMaxFloat;
+  empty_bounds(kp, empty, memp, false);
   kp.budget = tu.step_budget ? tu.step_budget : 32;
-  kp.refill_active = 32u - std::min<uint32_t>(tu.refill_idle ? tu.refill_idle : 32u, 32u);
-  kp.run_probe = tu.probe_in_run ? 1u : 0u;
-  kp.tail_share = std::min<uint32_t>(tu.tail_share, 32u);
-  // mix(c, c, t) three times stays within 12 roundings of c (relative 2^-24
-  // each); 0.999 leaves a wide margin
-  kp.empty_lo = empty ? 0.999f * e0.be * e0.min_scale : 0.0f;
-  // twelve roundings of 2^-24 stay far inside 2^-16
-  kp.empty_lo_t = e0.be * e0.min_scale * (1.0f - 1.52587890625e-5f);
-  kp.empty_hi = e0.be * e0.min_scale * (1.0f + 1.52587890625e-5f);
-  kp.settle_links = empty ? 48u : 0u;
+  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj);
+  kp.brute_field = c->empty_dist.as<uint8_t>();
   kp.plain_obj = (e0.m[12] == 0.0f && e0.m[13] == 0.0f && e0.m[14] == 0.0f && e0.min_scale == 1.0f) ? 1u : 0u;
   const void* fn = nullptr;
   switch (c->cfg.precision) {
@@ -2035,7 +1781,8 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
     bps = occ > 0 ? static_cast<uint32_t>(occ) : 1;
   }
   uint64_t blocks = static_cast<uint64_t>(c->sm_count) * bps;
-  const uint64_t need_blocks = (total + threads - 1) / threads;
+  const uint64_t block_rays = threads / 32 * detail::kLeastLanes;  // (lane_share spreads them)
+  const uint64_t need_blocks = (total + block_rays - 1) / block_rays;
   if (blocks > need_blocks) blocks = need_blocks ? need_blocks : 1;
   void* args[] = {&kp};
   rkf_status se = c->march_event(st, false);

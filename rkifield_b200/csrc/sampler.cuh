@@ -64,8 +64,11 @@ __device__ __forceinline__ uint32_t lookup_cached(const SceneDev& s, const ObjDe
 }
 
 // sample_voxelized (grad=false) / sample_voxelized_grad (grad=true) at an
-// object-local position.
-template <int PREC>
+// object-local position.  SIMPLE: an object of the empty-space path (verified
+// exact quotient, fewer than 2^20 voxels per axis), whose sampler needs
+// neither the IEEE quotient nor the wide floor: less code, and the march is
+// bound by fetching its code.
+template <int PREC, bool SIMPLE = false>
 __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, float lx, float ly,
                                             float lz, bool grad, LaneCache& lc) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]);
@@ -94,7 +97,7 @@ __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, 
     }
   }
   float qx, qy, qz;
-  if (o.div_ok) {
+  if (SIMPLE || o.div_ok) {
     qx = exact_div_vs(clx, o.vs, o.rcp_vs);
     qy = exact_div_vs(cly, o.vs, o.rcp_vs);
     qz = exact_div_vs(clz, o.vs, o.rcp_vs);
@@ -104,9 +107,15 @@ __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, 
     qz = __fdiv_rn(clz, o.vs);
   }
   const float vcx = __fsub_rn(qx, 0.5f), vcy = __fsub_rn(qy, 0.5f), vcz = __fsub_rn(qz, 0.5f);
-  const float fx = floorf(vcx), fy = floorf(vcy), fz = floorf(vcz);
-  const float tx = __fsub_rn(vcx, fx), ty = __fsub_rn(vcy, fy), tz = __fsub_rn(vcz, fz);
-  const int x0 = static_cast<int>(fx), y0 = static_cast<int>(fy), z0 = static_cast<int>(fz);
+  int x0, y0, z0;
+  float tx, ty, tz;
+  if (SIMPLE || max(o.tv[0], max(o.tv[1], o.tv[2])) < (1 << 21)) {
+    tx = floor_frac(vcx, x0), ty = floor_frac(vcy, y0), tz = floor_frac(vcz, z0);
+  } else {
+    const float fx = floorf(vcx), fy = floorf(vcy), fz = floorf(vcz);
+    tx = __fsub_rn(vcx, fx), ty = __fsub_rn(vcy, fy), tz = __fsub_rn(vcz, fz);
+    x0 = static_cast<int>(fx), y0 = static_cast<int>(fy), z0 = static_cast<int>(fz);
+  }
   // cl lies in [vs*0.01, grid - vs*0.01] (never NaN: the clamp maps NaN to a
   // bound), so the lower corner x0 is in [-1, tv-1]: clamping x0 from below
   // and x0+1 from above is the shader's two-sided clamp of both
@@ -216,8 +225,9 @@ __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, 
   return __fadd_rn(mixf(c0, c1, tz), outside);
 }
 
-// Nearest-voxel slot lookup of sample_voxelized_material / _blend_data.
-__device__ __forceinline__ uint32_t nearest_slot(const SceneDev& s, const ObjDev& o, float lx,
+// Nearest-voxel slot lookup of sample_voxelized_material / _blend_data.  (Out
+// of line, as everything that only hits need: see sample_vox.)
+static __device__ __noinline__ uint32_t nearest_slot(const SceneDev& s, const ObjDev& o, float lx,
                                                  float ly, float lz, uint32_t& idx, LaneCache& lc) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]);
   const float gpy = __fadd_rn(ly, o.half_gs[1]);

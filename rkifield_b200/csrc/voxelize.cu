@@ -523,7 +523,14 @@ extern "C" rkf_status rkf_voxelize_prims(rkf_ctx* ctx, const rkf_prim* prims, ui
     if (top_off) RKF_CUDA_TRY(cudaMemcpyAsync(nf.p, c->empty_dist.p, top_off, cudaMemcpyDeviceToDevice, c->stream));
     RKF_CUDA_TRY(cudaMemcpyAsync(nt.as<uint32_t>() + top_off, top.data(), ntop * 4, cudaMemcpyHostToDevice, c->stream));
     if ((st = build_empty_dist(od, nt.as<uint32_t>(), nf.as<uint8_t>(), c->stream)) != RKF_OK) return st;
-    c->counted(3);
+    std::vector<uint32_t> leaf_blocks;
+    leaf_blocks.reserve(n_new_leaves);
+    for (size_t b = 0; b < ntop; ++b)
+      if (top[b] < RKF_INTERIOR_SLOT) leaf_blocks.push_back(static_cast<uint32_t>(top_off + b));
+    if ((st = build_leaf_dist(od, nt.as<uint32_t>(), c->leaves.as<uint32_t>(), c->leaf_dist.as<uint8_t>(),
+                              leaf_blocks, c->stream)) != RKF_OK)
+      return st;
+    c->counted(leaf_blocks.empty() ? 3 : 4);
     std::swap(c->top.p, nt.p);
     std::swap(c->top.bytes, nt.bytes);
     std::swap(c->empty_dist.p, nf.p);
