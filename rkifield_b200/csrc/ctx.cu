@@ -639,6 +639,8 @@ rkf_status rkf_objects_import(rkf_ctx* ctx, const rkf_gpu_object* objects, uint3
   uint32_t cap = 64;
   while (cap < nl) cap *= 2;
   DevBuf nleaves, nleafd, ntop, nfield;
+  c->spare_top.release();  // (of the index this import replaces)
+  c->spare_field.release();
   rkf_status st = nleaves.alloc(static_cast<size_t>(cap) * 2048);
   if (st == RKF_OK) st = nleafd.alloc(static_cast<size_t>(cap) * 512);
   if (st == RKF_OK) st = ntop.alloc(std::max<size_t>(top.size(), 1) * 4);

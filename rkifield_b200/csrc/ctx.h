@@ -133,6 +133,11 @@ struct Ctx {
   cudaEvent_t band_ev[kMaxBands] = {};
   cudaEvent_t segs_ev = nullptr;
   DevBuf order_buf;  // heaviest-first tile order of views (tile_order.h)
+  // direct edits: the index of the epoch before, which the next edit writes its
+  // own into, and the edits' temporaries (at most kEditKept bytes stay)
+  static constexpr size_t kEditKept = 32u << 20;
+  DevBuf spare_top, spare_field;
+  std::vector<std::unique_ptr<DevBuf>> edit_bufs;
   DevBuf settle_buf; // lists of the settling passes (settle.h)
   DevBuf counters;   // work counters of the persistent kernels
   DevBuf seg_buf;    // segment table of the persistent kernel

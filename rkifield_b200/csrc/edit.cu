@@ -248,7 +248,7 @@ struct Temp {
   rkf_status get(const EditScratch* scratch, size_t bytes) {
     if (scratch) {
       p = (*scratch)(bytes);
-      return p ? RKF_OK : fail(RKF_OOM, "rkf_edit_csg: no scratch room for the edit");
+      return p ? RKF_OK : fail(RKF_OOM, "rkf_edit_csg: allocation of the edit's scratch failed");
     }
     rkf_status st = own.alloc(bytes);
     p = own.p;
@@ -528,13 +528,50 @@ extern "C" rkf_status rkf_edit_csg(rkf_ctx* ctx, const rkf_edit_op* op, uint64_t
   // direct edits: nothing else holds the old epoch once the context stream is idle
   RKF_CUDA_TRY(cudaStreamSynchronize(c->stream));
   EditOutcome r;
-  rkf_status st = apply_edit(c, *op, c->stream, &r);
+  // The index of two epochs back is this edit's to write: what read it ended
+  // before the last edit returned (the wait at the end).  Allocating and freeing
+  // an index (43 MB over the 1.1M-brick scene) and the temporaries on each edit
+  // took most of it.
+  if (c->spare_top.p && c->spare_top.bytes == std::max<uint64_t>(c->top_len, 1) * 4 &&
+      c->spare_field.bytes == std::max<uint64_t>(c->top_len, 1)) {
+    r.top_dst = c->spare_top.as<uint32_t>();
+    r.field_dst = c->spare_field.as<uint8_t>();
+  } else {
+    c->spare_top.release();
+    c->spare_field.release();
+  }
+  size_t next_buf = 0, kept = 0;
+  const EditScratch scratch = [&](size_t bytes) -> void* {
+    // a buffer per temporary, in the order an edit asks for them
+    if (next_buf == c->edit_bufs.size()) c->edit_bufs.push_back(std::make_unique<DevBuf>());
+    DevBuf& b = *c->edit_bufs[next_buf];
+    if (b.bytes < bytes && b.alloc(bytes + bytes / 4) != RKF_OK) return nullptr;
+    ++next_buf;
+    return b.p;
+  };
+  rkf_status st = apply_edit(c, *op, c->stream, &r, &scratch);
+  // marches of the old epoch on other streams end before its index is spare,
+  // and error paths may return with work queued
+  RKF_CUDA_TRY(cudaDeviceSynchronize());
+  for (size_t i = 0; i < c->edit_bufs.size(); ++i)
+    if ((kept += c->edit_bufs[i]->bytes) > Ctx::kEditKept) {
+      c->edit_bufs.resize(i);
+      break;
+    }
   if (st != RKF_OK) return st;
-  if (r.new_top.p) {
-    std::swap(c->top.p, r.new_top.p);
-    std::swap(c->top.bytes, r.new_top.bytes);
-    std::swap(c->empty_dist.p, r.new_empty_dist.p);
-    std::swap(c->empty_dist.bytes, r.new_empty_dist.bytes);
+  if (r.new_epoch) {
+    DevBuf& top = r.new_top.p ? r.new_top : c->spare_top;
+    DevBuf& field = r.new_top.p ? r.new_empty_dist : c->spare_field;
+    std::swap(c->top.p, top.p);
+    std::swap(c->top.bytes, top.bytes);
+    std::swap(c->empty_dist.p, field.p);
+    std::swap(c->empty_dist.bytes, field.bytes);
+    if (r.new_top.p) {  // the old epoch's index becomes the spare one
+      std::swap(c->spare_top.p, r.new_top.p);
+      std::swap(c->spare_top.bytes, r.new_top.bytes);
+      std::swap(c->spare_field.p, r.new_empty_dist.p);
+      std::swap(c->spare_field.bytes, r.new_empty_dist.bytes);
+    }
     c->epoch++;
     for (uint32_t s : r.retired) c->free_slots.push_back(s);
     for (uint32_t l : r.retired_leaves) c->free_leaves.push_back(l);
