@@ -441,6 +441,18 @@ rkf_status rkf_create(const rkf_config* cfg, rkf_ctx** out) {
   // room for the settling passes of a 1920x1080 view, so that a first view does
   // not wait for it; larger ones grow it, and without it views march alone
   if (c->settle_buf.alloc(settle_bytes(1920u * 1080u, 32)) != RKF_OK) cudaGetLastError();
+  void *hs = nullptr, *hd = nullptr;
+  if (cudaHostAlloc(&hs, Ctx::kHostStage, cudaHostAllocMapped) == cudaSuccess) {
+    if (cudaHostGetDevicePointer(&hd, hs, 0) == cudaSuccess) {
+      c->host_stage = static_cast<char*>(hs);
+      c->host_stage_dev = static_cast<char*>(hd);
+    } else {
+      cudaGetLastError();
+      cudaFreeHost(hs);
+    }
+  } else {
+    cudaGetLastError();
+  }
   c->free_slots.resize(cap);
   for (size_t i = 0; i < cap; ++i) c->free_slots[i] = static_cast<uint32_t>(cap - 1 - i);
   c->tuning = rkf_batch_tuning{4, 8, 32, 64, 0, 256, 32, 0, 0};
@@ -466,6 +478,7 @@ rkf_status rkf_destroy(rkf_ctx* ctx) {
     if (e) cudaEventDestroy(e);
   if (c->segs_ev) cudaEventDestroy(c->segs_ev);
   for (cudaEvent_t e : c->march_ev) cudaEventDestroy(e);
+  if (c->host_stage) cudaFreeHost(c->host_stage);
   delete c;
   return RKF_OK;
 }

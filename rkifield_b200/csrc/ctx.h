@@ -124,6 +124,11 @@ struct Ctx {
 
   // scratch reused by march calls (host-pointer outputs staged here)
   DevBuf stage;
+  // page-locked host memory that kernels of small host-pointer calls read and
+  // write in place (null: none could be had)
+  static constexpr size_t kHostStage = 512u << 10;
+  char* host_stage = nullptr;      // as the host sees it
+  char* host_stage_dev = nullptr;  // as the device sees it
   // host-output views: band b marches on band_stream[b % 2] (so a band's
   // launch fills the SMs its predecessor's last rays leave idle), and its
   // rows go back on copy_stream once band_ev[b] has completed
