@@ -109,7 +109,7 @@ __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, 
   const float vcx = __fsub_rn(qx, 0.5f), vcy = __fsub_rn(qy, 0.5f), vcz = __fsub_rn(qz, 0.5f);
   int x0, y0, z0;
   float tx, ty, tz;
-  if (SIMPLE || max(o.tv[0], max(o.tv[1], o.tv[2])) < (1 << 21)) {
+  if (SIMPLE) {  // (fewer than 2^20 voxels an axis)
     tx = floor_frac(vcx, x0), ty = floor_frac(vcy, y0), tz = floor_frac(vcz, z0);
   } else {
     const float fx = floorf(vcx), fy = floorf(vcy), fz = floorf(vcz);
