@@ -1084,6 +1084,16 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
   }
 }
 
+// The object table into shared memory, a word a thread (a record of some 400
+// bytes a thread cost a block of a small scene as long as a sample).
+__device__ __forceinline__ void load_objs(ObjDev* sh, const SceneDev& s) {
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(s.objs);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(sh);
+  static_assert(sizeof(ObjDev) % 4 == 0, "whole words");
+  for (uint32_t i = threadIdx.x; i < s.n_objs * static_cast<uint32_t>(sizeof(ObjDev) / 4); i += blockDim.x)
+    dst[i] = __ldg(src + i);
+}
+
 constexpr uint32_t kPointLanes = 8;
 
 // SdfQueryable::evaluate / gradient over the pool, eight lanes a point: each
@@ -1098,7 +1108,7 @@ template <int PREC>
 __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* __restrict__ pts, uint32_t n,
                                                      float* dist, float* grad, uint16_t* material) {
   extern __shared__ ObjDev sh_objs[];
-  for (uint32_t i = threadIdx.x; i < s.n_objs; i += blockDim.x) sh_objs[i] = s.objs[i];
+  load_objs(sh_objs, s);
   __syncthreads();
   const uint32_t id = blockIdx.x * (blockDim.x / kPointLanes) + threadIdx.x / kPointLanes;
   const uint32_t j = threadIdx.x % kPointLanes;
@@ -1213,7 +1223,7 @@ template <int PREC>
 __global__ void k_sdf_ao(SceneDev s, const float* __restrict__ pos, const float* __restrict__ nrm, uint32_t n,
                          float* __restrict__ ao) {
   extern __shared__ ObjDev sh_objs[];
-  for (uint32_t i = threadIdx.x; i < s.n_objs; i += blockDim.x) sh_objs[i] = s.objs[i];
+  load_objs(sh_objs, s);
   __syncthreads();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
