@@ -576,17 +576,17 @@ typedef struct rkf_batch_tuning {
     uint32_t tile_w, tile_h;     /* ray-tile shape of a work item            */
     uint32_t step_budget;        /* empty-space steps a lane runs before its */
                                  /* warp re-converges (0 = 32)               */
-    uint32_t compact_interval;   /* march iterations between lane refills;   */
-                                 /* a warp also refills once refill_idle of  */
-                                 /* its lanes are done (0 = 64)              */
+    uint32_t compact_interval;   /* phases a warp takes between lane refills */
+                                 /* at most, once any of its lanes is done;  */
+                                 /* it also refills once refill_idle of them */
+                                 /* are (0 = 64)                             */
     uint32_t blocks_per_sm;
     uint32_t threads_per_block;
-    uint32_t refill_idle;        /* a warp leaves the march loop to refill   */
-                                 /* once this many of its lanes are idle     */
-                                 /* (0 = 32: only when all are idle)         */
-    uint32_t probe_in_run;       /* 1: a lane whose EMPTY cube ends probes   */
-                                 /* the next one inside the run (0: at the   */
-                                 /* run's end, with the warp's other lanes)  */
+    uint32_t refill_idle;        /* a warp takes new rays once this many of  */
+                                 /* its lanes are done (0 or 32: the kernel's */
+                                 /* own choice)                              */
+    uint32_t probe_in_run;       /* 0 or 1; without effect: walks are a      */
+                                 /* phase of their own                       */
     uint32_t no_empty_path;      /* 1: march every step through the full     */
                                  /* sampler (0: EMPTY runs wherever the      */
                                  /* scene allows them).  rkf_march,          */
@@ -594,15 +594,12 @@ typedef struct rkf_batch_tuning {
                                  /* the outputs are the same either way      */
     uint32_t order_tiles;        /* 1: hand out each view's ray tiles        */
                                  /* heaviest first, by an estimate of their  */
-                                 /* empty-space steps (0: row order); the    */
+                                 /* empty-space steps (0: row order).  Views */
+                                 /* large enough to have their misses        */
+                                 /* settled before the march go without; the */
                                  /* outputs are the same either way          */
-    uint32_t tail_share;         /* once a warp has no work left to fetch    */
-                                 /* and at most this many of its lanes still */
-                                 /* march (1..32), the warp's 32 lanes take  */
-                                 /* those lanes' EMPTY runs together, one    */
-                                 /* run at a time, up to 32 steps a round;   */
-                                 /* 0: off.  Single-object empty-space path; */
-                                 /* the outputs are the same either way      */
+    uint32_t tail_share;         /* 0..32; without effect: the last rays are */
+                                 /* spread over the chip's warps             */
 } rkf_batch_tuning;
 
 /* Run every view and ray batch in one persistent work-stealing launch.

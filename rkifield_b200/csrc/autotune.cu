@@ -1,19 +1,16 @@
 // autotune.cu — pick the persistent march's launch tuning for a workload.
 //
-// The batched march has nine knobs that change speed but never results:
+// The batched march has seven knobs that change speed but never results:
 // the ray-tile shape that orders a view's work ids (the spatial coherence of
-// the rays a warp holds), the compaction interval (march iterations between
-// lane refills), the step budget (empty-space steps a lane runs before its
+// the rays a warp holds), the compaction interval (phases between lane
+// refills), the step budget (empty-space steps a lane runs before its
 // warp re-converges), the refill threshold (idle lanes that make a warp
-// refill), where a lane probes its next EMPTY cube (inside a run or between
-// runs), the block size, whether it runs EMPTY runs at all, whether views
-// hand out their heaviest ray tiles first and whether the warps of the
-// launch's tail share their EMPTY runs.  rkf_autotune times candidates on
+// refill), the block size, whether it runs EMPTY runs at all and whether views
+// hand out their heaviest ray tiles first.  rkf_autotune times candidates on
 // the caller's sample of the work with CUDA events: every tile x interval x
 // block size at the default budget and threshold, then the heaviest-first
-// tile order, then every budget, then every threshold, then the other probe
-// placement, then warp-shared EMPTY runs in the launch's tail, then the march
-// without EMPTY runs, each at the best so far.
+// tile order, then every budget, then every threshold, then the march without
+// EMPTY runs, each at the best so far.
 // Each timed launch starts with the L2 cache flushed (a write of twice its
 // size, outside the timed events), as a frame does after other work: with
 // the index left in L2 by the previous trial, the knobs that cut DRAM
@@ -108,17 +105,6 @@ extern "C" rkf_status rkf_autotune(rkf_ctx* ctx, const rkf_view* views, uint32_t
     if (st != RKF_OK) break;
     rkf_batch_tuning tu = base2;
     tu.refill_idle = r;
-    trial(tu);
-  }
-  if (st == RKF_OK) {
-    rkf_batch_tuning tu = best;
-    tu.probe_in_run = 1;
-    trial(tu);
-  }
-  // the warp-shared EMPTY runs of the launch's tail
-  if (st == RKF_OK) {
-    rkf_batch_tuning tu = best;
-    tu.tail_share = 2;
     trial(tu);
   }
   // where EMPTY runs do not pay (a camera outside a dense grid: short runs,
