@@ -1095,6 +1095,7 @@ __device__ __forceinline__ void load_objs(ObjDev* sh, const SceneDev& s) {
 }
 
 constexpr uint32_t kPointLanes = 8;
+constexpr uint32_t kAoLanes = 4;  // one per tap
 
 // SdfQueryable::evaluate / gradient over the pool, eight lanes a point: each
 // evaluates its share of the objects, then six of them one sample of the
@@ -1102,8 +1103,8 @@ constexpr uint32_t kPointLanes = 8;
 // itself.  All samples go through one copy of the evaluator.  A thread per point
 // took its 7 samples one after the other, through a copy each (246 KB of code):
 // bound by instruction fetch and by that chain, 54 us for 300 points near
-// surfaces (20 so) and 66 us for 65,536 over the 1.1M-brick scene (61; there the
-// bound is the samples' loads, which this order leaves as they are).
+// surfaces (20 so) and, as a call, 72 us for 65,536 over the 1.1M-brick scene (56
+// so; there the bound is the samples' loads).
 template <int PREC>
 __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* __restrict__ pts, uint32_t n,
                                                      float* dist, float* grad, uint16_t* material) {
@@ -1214,35 +1215,44 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
   grad[3 * static_cast<size_t>(i) + 2] = nz;
 }
 
-// One thread per point: sdf_ao (shade_common_shading.wgsl:37-47), four taps
-// along the normal at AO_STEP_SIZE * i (0.12 m) through sample_sdf, which for
-// points inside the objects' bounds is the minimum of evaluate_object over the
-// objects (shade_common.wgsl:521-572); ao = clamp(1 - AO_STRENGTH * sum, 0, 1)
-// with AO_STRENGTH 0.7 and tap weights 1, 1/2, 1/4, 1/8.
+// sdf_ao (shade_common_shading.wgsl:37-47), four taps along the normal at
+// AO_STEP_SIZE * i (0.12 m) through sample_sdf, which for points inside the
+// objects' bounds is the minimum of evaluate_object over the objects
+// (shade_common.wgsl:521-572); ao = clamp(1 - AO_STRENGTH * sum, 0, 1) with
+// AO_STRENGTH 0.7 and tap weights 1, 1/2, 1/4, 1/8.
+// A lane per tap, added up in the taps' order: bound by the chain of a tap's
+// loads, of which a thread per point took four in a row.  Call times over the
+// 32 m scene, 64 / 30,000 / 200,003 / 500,000 points: 32 / 35 / 58 / 86 us for a
+// thread per point, 19 / 21 / 44 / 81 us so; 12 blocks an SM (40 registers), as
+// 10 take 46 and 85 for the last two.
 template <int PREC>
-__global__ void k_sdf_ao(SceneDev s, const float* __restrict__ pos, const float* __restrict__ nrm, uint32_t n,
-                         float* __restrict__ ao) {
+__global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __restrict__ pos,
+                                                   const float* __restrict__ nrm, uint32_t n,
+                                                   float* __restrict__ ao) {
   extern __shared__ ObjDev sh_objs[];
   load_objs(sh_objs, s);
   __syncthreads();
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const uint64_t id = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kAoLanes;
+  const uint32_t k = 1u + threadIdx.x % kAoLanes;
+  const uint32_t i = id < n ? static_cast<uint32_t>(id) : n - 1u;  // (every lane takes part in the exchange)
   LaneCache lc;
   const size_t i3 = 3 * static_cast<size_t>(i);
   const float px = pos[i3], py = pos[i3 + 1], pz = pos[i3 + 2];
   const float nx = nrm[i3], ny = nrm[i3 + 1], nz = nrm[i3 + 2];
+  const float dist = __fmul_rn(0.12f, static_cast<float>(k));
+  float du;
+  uint32_t bi;
+  const float d = eval_min<PREC, false>(s, sh_objs, 0, s.n_objs, __fadd_rn(px, __fmul_rn(nx, dist)),
+                                       __fadd_rn(py, __fmul_rn(ny, dist)), __fadd_rn(pz, __fmul_rn(nz, dist)), du,
+                                       bi, lc);
+  const float tap = __fsub_rn(dist, d);
   float acc = 0.0f, scale = 1.0f;
-#pragma unroll 1
-  for (uint32_t k = 1; k <= 4; ++k) {
-    const float dist = __fmul_rn(0.12f, static_cast<float>(k));
-    float du;
-    uint32_t bi;
-    const float d = eval_min<PREC, false>(s, sh_objs, 0, s.n_objs, __fadd_rn(px, __fmul_rn(nx, dist)),
-                                         __fadd_rn(py, __fmul_rn(ny, dist)), __fadd_rn(pz, __fmul_rn(nz, dist)), du,
-                                         bi, lc);
-    acc = __fadd_rn(acc, __fmul_rn(scale, __fsub_rn(dist, d)));
+#pragma unroll
+  for (int a = 0; a < static_cast<int>(kAoLanes); ++a) {  // in the taps' order
+    acc = __fadd_rn(acc, __fmul_rn(scale, __shfl_sync(kFull, tap, a, kAoLanes)));
     scale = __fmul_rn(scale, 0.5f);
   }
+  if (id >= n || k != 1u) return;
   ao[i] = clampf(__fsub_rn(1.0f, __fmul_rn(0.7f, acc)), 0.0f, 1.0f);
 }
 
@@ -1877,7 +1887,7 @@ rkf_status launch_query(Ctx* c, const float* pts, uint32_t n, float* d, float* g
 rkf_status launch_ao(Ctx* c, const float* pos, const float* nrm, uint32_t n, float* ao, cudaStream_t st) {
   if (n == 0) return RKF_OK;
   const size_t smem = sizeof(ObjDev) * std::max<uint32_t>(1, c->obj_count());
-  const unsigned blocks = (n + 127) / 128;
+  const unsigned blocks = (n - 1) / (128 / detail::kAoLanes) + 1;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
       detail::k_sdf_ao<RKF_PRECISION_F32><<<blocks, 128, smem, st>>>(c->scene_dev(), pos, nrm, n, ao);

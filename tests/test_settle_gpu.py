@@ -164,6 +164,18 @@ def test_point_counts_agree(small_scene, n_objs):
         ctx.close()
 
 
+def test_occlusion_counts_agree(one):
+    """The taps of a point are lanes of one warp: block edges (32 points)."""
+    rng = np.random.default_rng(8)
+    pos = rng.uniform(-16.0, 16.0, (5000, 3)).astype(np.float32)
+    nrm = rng.standard_normal((5000, 3))
+    nrm = (nrm / np.linalg.norm(nrm, axis=1, keepdims=True)).astype(np.float32)
+    ao = one.sdf_ao(pos, nrm)
+    assert 0.0 <= ao.min() < 1.0
+    for n in (1, 7, 8, 9, 31, 32, 33, 4097):
+        assert_bits_equal(one.sdf_ao(pos[-n:], nrm[-n:]), ao[-n:], str(n))
+
+
 @pytest.mark.parametrize("size", [(1, 1), (37, 11), (64, 8)])
 def test_secondary_rays_per_pixel(one, small_scene, size):
     """Each ray of a call with several lights and occlusion rays is the ray of the
