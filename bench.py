@@ -996,7 +996,7 @@ def run_b200(args, world, rank, local, dist):
 
     def timed(plain: bool, steps: int, warmup: int):
         """Step times (events around the whole call: tile order + march), the
-        march kernel's own times (events around its launch alone), the
+        march's own times (events around the settling passes and it), the
         library's kernel launches in the timed region and the wall time."""
         for _ in range(warmup):
             ctx.march_async(cam, p, w, h, gp, stream.ptr, plain=plain)
@@ -1105,7 +1105,7 @@ def run_b200(args, world, rank, local, dist):
                         "steps_per_ray": st["steps"] / st["rays"],
                         "sample_rows": args.sector_rows,
                         "kernel_ms": mean_s * 1e3,
-                        "kernel_timing": ("CUDA events around the march kernel's launch alone"
+                        "kernel_timing": ("CUDA events around the settling passes and the march"
                                           if kernel_ms else "CUDA events around the step")}
             if not args.no_cpu:
                 rows = sample_rows(h, args.cpu_rows)
@@ -1138,7 +1138,7 @@ def run_b200(args, world, rank, local, dist):
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
             "gpu_launches": launches,
-            "gpu_launches_note": "kernels the library launched in the timed region (march + tile order), "
+            "gpu_launches_note": "kernels the library launched in the timed region (settling passes + march), "
                                  "counted by the context",
             "wall_s_timed_region": wall,
         }

@@ -1745,6 +1745,9 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   // against 1.0.
   const bool few = empty && few_empty_steps(kp, multi_empty, tiled ? kFewStepsTiled : kFewSteps);
   const bool tiled_empty = tiled && empty;
+  // (march timing covers the passes too)
+  rkf_status se = c->march_event(st, false);
+  if (se != RKF_OK) return se;
   if (settle && empty && (!tiled_empty || few)) {
     const size_t need = settle_bytes(view_ids, kp.tile_w * kp.tile_h);
     if (c->settle_buf.bytes >= need || c->settle_buf.alloc(need + need / 8) == RKF_OK) {
@@ -1781,8 +1784,6 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   const uint64_t need_blocks = (total + block_rays - 1) / block_rays;
   if (blocks > need_blocks) blocks = need_blocks ? need_blocks : 1;
   void* args[] = {&kp};
-  rkf_status se = c->march_event(st, false);
-  if (se != RKF_OK) return se;
   RKF_CUDA_TRY(cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(threads), args, smem, st));
   c->counted();
   return c->march_event(st, true);
