@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(128) k_settle_tiles(const __grid_constant__ KP
     const float r = (sqrtf(rr) * static_cast<float>(kp.tile_w) / static_cast<float>(sg.w) +
                      sqrtf(uu) * static_cast<float>(kp.tile_h) / static_cast<float>(sg.h)) * 1.0001f;
     const float spread = r / (len - r) * 1.0001f + 4.0e-6f;
-    if (len > 2.0f * r && spread < 0.25f) {
+    if (len > 2.0f * r && len < kMaxRate && spread < 0.25f) {  // (a finite camera)
       // one walk per voxelized object of the path
       const uint32_t n_ev = SINGLE ? 1u : kp.n_ev;
       bool ok = true, exact = false;

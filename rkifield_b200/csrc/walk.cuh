@@ -295,10 +295,13 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // where it enters and at (x - 2 margin) * inv - cin where it leaves.  margin
 // covers every rounding between t and the sampler's grid coordinate and every
 // rounding made here: 0.1 voxel plus 2^-18 of the magnitudes involved, a wide
-// multiple of the few 2^-24 roundings.
+// multiple of the few 2^-24 roundings.  It is infinite for a direction that is
+// NaN, infinite or beyond kMaxRate voxels per unit of t, of which face times say
+// nothing (the reciprocal underflows to zero): no walk starts then.
 struct ProbeRay {
   float g[3], d[3], inv[3], cin[3], margin;
 };
+constexpr float kMaxRate = 1.152921504606847e18f;  // 2^60
 
 __device__ __forceinline__ int down_mask(const ProbeRay& r, int a) { return __float_as_int(r.d[a]) >> 31; }
 __device__ __forceinline__ float mirrored(const ObjDev& o, const ProbeRay& r, int a, float v) {
@@ -313,6 +316,9 @@ __device__ __forceinline__ ProbeRay probe_ray(const ObjDev& o, float ox, float o
 #pragma unroll
   for (int a = 0; a < 3; ++a) mag += fabsf(og[a]) + o.mag[a];
   r.margin = 0.1f + mag * o.rcp_vs * 3.814697265625e-6f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    if (!(fabsf(dir[a]) * o.rcp_vs <= kMaxRate)) r.margin = INFINITY;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     r.g[a] = (og[a] + o.m[12 + a] + o.half_gs[a]) * o.rcp_vs - 0.5f;
@@ -386,7 +392,8 @@ __device__ __forceinline__ bool walk_start(const ObjDev& o, const SceneDev& s, c
 #pragma unroll
   for (int a = 0; a < 3; ++a) out[a] = A.out[a];
   end = fminf(fminf(A.out[0], A.out[1]), A.out[2]);
-  // (a margin beyond two voxels: a seam would span more than a brick)
+  // (a margin beyond two voxels, or none that would do: a seam would span more
+  // than a brick)
   return fmaxf(fmaxf(A.in[0], A.in[1]), A.in[2]) <= t && end >= t && r.margin < 2.0f;
 }
 
