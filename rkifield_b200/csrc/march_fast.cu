@@ -691,14 +691,11 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
       // and it is settled here.  Otherwise the walk's end bounds the run.
       if (walk) {
         uint32_t outcome = 0;  // 1: ends past tmax; 2: runs out of steps
-        // t after k more steps lies in [t + k*lo, t + k*hi] widened by one
-        // rounding (2^-24) per step; 2^-22 per step (and 4 more) leaves room
-        // for this bound's own rounding.  The last sample is the
-        // (max_step-step-1)th ahead: the ray ends past tmax (with no step
-        // flag) if even its smallest t exceeds tmax by then, and runs out of
-        // steps if even its largest t stays <= tmax.
+        // The last sample is the (max_step-step-1)th ahead: the ray ends past
+        // tmax (with no step flag) if even its smallest t exceeds tmax by then,
+        // and runs out of steps if even its largest t stays <= tmax.
         const float k = static_cast<float>(max_step - step - 1);
-        const float grow = (k + 4.0f) * 2.384185791015625e-7f;
+        const float grow = steps_grow(k);
         const float t_lo = (t + k * kp.empty_lo_t) * (1.0f - grow);
         const float t_hi = (t + k * kp.empty_hi) * (1.0f + grow);
         const bool can = kp.empty_lo >= brk && kp.empty_lo >= near_thr && kp.empty_lo >= min_step;

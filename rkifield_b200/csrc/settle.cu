@@ -146,13 +146,19 @@ __device__ __forceinline__ bool thresholds_clear(const KParams& kp) {
          kp.empty_lo >= p.min_step && p.scene.max_steps > 0u && p.hard_max_steps > 0u && p.scene.max_distance >= 0.0f;
 }
 
-// kSingle: one voxelized object, brute strategy (or its equal); else any scene
+// The latest the last step can begin.
+__device__ __forceinline__ float last_step(const KParams& kp) {
+  const float k = static_cast<float>(kp.p.hard_max_steps - 1u);
+  return k * kp.empty_hi * (1.0f + steps_grow(k));
+}
+
+// SINGLE: one voxelized object, brute strategy (or its equal); else any scene
 // and strategy of the empty-space path (tiled launches only past tmax).
 template <bool SINGLE>
 __device__ __forceinline__ Ending tile_ending(const KParams& kp, const Beam& b, const ObjDev& o) {
   const float k = static_cast<float>(kp.p.hard_max_steps - 1u), tmax = kp.p.scene.max_distance;
-  const float grow = (k + 4.0f) * 2.384185791015625e-7f;
-  const float t_lo = k * kp.empty_lo_t * (1.0f - grow), t_hi = k * kp.empty_hi * (1.0f + grow);
+  const float grow = steps_grow(k);
+  const float t_lo = k * kp.empty_lo_t * (1.0f - grow), t_hi = last_step(kp);
   if (t_lo > tmax) return {1u, tmax};
   if (kp.tiled) return {0u, 0.0f};
   // the whole beam in the core interval (core_interval), and past the clamp box
@@ -180,10 +186,10 @@ __device__ __forceinline__ Ending tile_ending(const KParams& kp, const Beam& b, 
   // leaves_grid, from t = 0, for every ray of the beam
   c *= o.min_scale * 0.998f;
   const float most =
-      __fdividef(fmaxf(t_o, 0.0f), kp.empty_lo_t) + __fdividef(2.0f, c) +
+      __fdividef(fmaxf(t_o * (1.0f + 2.0f * grow), 0.0f), kp.empty_lo_t) + __fdividef(2.0f, c) +
       __fdividef(__logf(fmaxf(__fdividef((tmax - t_o) * c, kp.empty_lo_t), 1.0f)), __logf(1.0f + c)) * 1.001f + 7.0f;
   if (most < k) return {1u, tmax};
-  if (core && t_out < tmax && floorf(t_out / kp.empty_hi) - 2.0f >= k) return {2u, tmax};
+  if (core && t_out < tmax && floorf(t_out * (1.0f - grow) / kp.empty_hi) - 2.0f >= k) return {2u, tmax};
   return {0u, 0.0f};
 }
 
@@ -241,8 +247,7 @@ __global__ void __launch_bounds__(128) k_settle_tiles(const __grid_constant__ KP
         // several objects: out of steps needs one whose steps are exact so far
         exact = exact || here.kind != 0u;
         if (!SINGLE && here.kind) end = here;
-        const float target = SINGLE || end.kind ? end.target
-                             : kp.tiled ? -1.0f : static_cast<float>(kp.p.hard_max_steps - 1u) * kp.empty_hi * 1.001f;
+        const float target = SINGLE || end.kind ? end.target : kp.tiled ? -1.0f : last_step(kp);
         ok = target >= 0.0f && beam_walk(o, kp.s, kp.brute_field, b, target, kp.walk_links);
       }
       ok = ok && exact && end.kind;
@@ -301,8 +306,7 @@ __global__ void __launch_bounds__(256) k_settle_rays(const __grid_constant__ KPa
         view_ray(sg, px, py, dx, dy, dz);
         dx = safe_dir(dx), dy = safe_dir(dy), dz = safe_dir(dz);
         const float k = static_cast<float>(kp.p.hard_max_steps - 1u);
-        const float grow = (k + 4.0f) * 2.384185791015625e-7f;
-        const float t_lo = k * kp.empty_lo_t * (1.0f - grow), t_hi = k * kp.empty_hi * (1.0f + grow);
+        const float t_lo = k * kp.empty_lo_t * (1.0f - steps_grow(k)), t_hi = last_step(kp);
         if (SINGLE) {
           const ObjDev& o = kp.objs[0];
           const ProbeRay r = probe_ray(o, sg.pos[0], sg.pos[1], sg.pos[2], dx, dy, dz);

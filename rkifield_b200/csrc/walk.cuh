@@ -488,6 +488,13 @@ __device__ __forceinline__ bool core_interval(const ObjDev& o, const ProbeRay& r
   return t >= t_in && t <= t_out;
 }
 
+// Where a ray is after n <= k steps of [lo, hi] each: each sum rounds by at most
+// 2^-24 of t, so t lies between (t + n lo) (1 - grow) and (t + n hi) (1 + grow)
+// (2^-22 a step, and 4 more, leaves room for these bounds' own rounding).
+// Turned round, t is surely at most T while t + n hi <= T (1 - grow), and at least
+// T from t + n lo >= T (1 + 2 grow) on (grow <= 1/2: at most 2^20 steps).
+__device__ __forceinline__ float steps_grow(float k) { return (k + 4.0f) * 2.384185791015625e-7f; }
+
 // How a ray whose every sample ahead is at least the EMPTY value ends when it
 // leaves the grid before it could run out of steps (one voxelized object): 1
 // past tmax, 2 out of steps, 0 undecided.  The ray runs out of steps exactly
@@ -522,15 +529,16 @@ __device__ __forceinline__ uint32_t leaves_grid(const ObjDev& o, const ProbeRay&
     }
   }
   c *= o.min_scale * 0.998f;
+  const float grow = steps_grow(k);
   const float most =
-      __fdividef(fmaxf(t_o - t, 0.0f), lo) + __fdividef(2.0f, c) +
+      __fdividef(fmaxf(t_o * (1.0f + 2.0f * grow) - t, 0.0f), lo) + __fdividef(2.0f, c) +
       __fdividef(__logf(fmaxf(__fdividef((tmax - t_o) * c, lo), 1.0f)), __logf(1.0f + c)) * 1.001f + 7.0f;
   if (most < k) return 1u;
   if (!core || !(t_out < tmax)) return 0u;
-  const float n0 = fmaxf(floorf(__fdividef(t_out - t, hi)) - 3.0f, 0.0f);
+  const float n0 = fmaxf(floorf(__fdividef(t_out * (1.0f - grow) - t, hi)) - 3.0f, 0.0f);
   if (n0 >= k) return 2u;
-  float L = (t + n0 * lo) * (1.0f - (n0 + 4.0f) * 2.384185791015625e-7f);
-  float U = (t + n0 * hi) * (1.0f + (n0 + 4.0f) * 2.384185791015625e-7f);
+  float L = (t + n0 * lo) * (1.0f - steps_grow(n0));
+  float U = (t + n0 * hi) * (1.0f + steps_grow(n0));
   const float be = o.be, be2 = o.be2, e_lo = be * (1.0f - 1.52587890625e-5f), e_hi = be * (1.0f + 1.52587890625e-5f);
   const float wide = 2.44140625e-4f, slack = r.margin * o.vs;
   float n = k - n0;
