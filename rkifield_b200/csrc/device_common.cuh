@@ -31,7 +31,10 @@ constexpr float kMaxFloat = 3.402823e+38f;  // ray_march.wgsl:27
 // Index: per object a top grid over 8^3-brick blocks (u32: EMPTY, INTERIOR or
 // a leaf number) and leaves of 512 u32 slots in x+8y+64z brick order.
 
-struct ObjDev {
+// What a sample of an object reads.  Kernels that copy the object table to
+// shared memory copy these records alone: 198 of them fit the 48 KB a launch
+// may ask for.
+struct ObjSample {
   float m[16];          // inverse_world, column-major
   float vs, be, be2;    // voxel size, brick extent, 2*brick extent
   float gs[3];          // grid size = dims * be
@@ -54,6 +57,10 @@ struct ObjDev {
   uint32_t div_ok;      // 1: exact_div_vs == IEEE x/vs verified on [lo, max(hi)]
   uint32_t translate_only;  // inverse_world is identity in its linear part
   float vs2;            // vs * 2 (INTERIOR value of the stepping sampler)
+};
+constexpr uint32_t kMaxObjectsShared = 49152 / sizeof(ObjSample);
+
+struct ObjDev : ObjSample {
   float last[3];        // tv - 1
   // the walk through EMPTY boxes, in voxel-centre coordinates: 2^n - 1 >= every
   // voxel index (at least 63; index v mirrors to v ^ mirror), the grid's border
@@ -129,7 +136,7 @@ __device__ __forceinline__ float f16_load(const uint16_t* p) {
 }
 
 // world -> object-local: r_i = ((m0i*x + m1i*y) + m2i*z) + m3i*1
-__device__ __forceinline__ void to_local(const ObjDev& o, float wx, float wy, float wz,
+__device__ __forceinline__ void to_local(const ObjSample& o, float wx, float wy, float wz,
                                          float& lx, float& ly, float& lz) {
   lx = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(o.m[0], wx), __fmul_rn(o.m[4], wy)),
                            __fmul_rn(o.m[8], wz)), __fmul_rn(o.m[12], 1.0f));
@@ -140,7 +147,7 @@ __device__ __forceinline__ void to_local(const ObjDev& o, float wx, float wy, fl
 }
 
 // analytic primitives (ray_march.wgsl:182-264)
-__device__ __forceinline__ float analytic_sdf(const ObjDev& o, float x, float y, float z) {
+__device__ __forceinline__ float analytic_sdf(const ObjSample& o, float x, float y, float z) {
   const float a0 = o.params[0], a1 = o.params[1], a2 = o.params[2];
   switch (o.prim_type) {
     case RKF_PRIM_SPHERE:
@@ -178,12 +185,12 @@ __device__ __forceinline__ float analytic_sdf(const ObjDev& o, float x, float y,
 // ---------------------------------------------------------------------------
 // Index lookup
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t top_index(const ObjDev& o, uint32_t bx, uint32_t by,
+__device__ __forceinline__ uint32_t top_index(const ObjSample& o, uint32_t bx, uint32_t by,
                                               uint32_t bz) {
   return o.top_off + (bx >> 3) + (by >> 3) * o.tdim[0] + (bz >> 3) * o.tdim[0] * o.tdim[1];
 }
 
-__device__ __forceinline__ uint32_t lookup2(const SceneDev& s, const ObjDev& o, uint32_t bx,
+__device__ __forceinline__ uint32_t lookup2(const SceneDev& s, const ObjSample& o, uint32_t bx,
                                             uint32_t by, uint32_t bz) {
   const uint32_t t = __ldg(s.top + top_index(o, bx, by, bz));
   if (t >= RKF_INTERIOR_SLOT) return t;

@@ -121,31 +121,6 @@ __device__ __forceinline__ float eval_bvh(const SceneDev& s, const ObjDev* objs,
 }
 
 
-// Minimum over objects [ob, oe) of evaluate_object at world position q.
-// SINGLE: the scene is exactly one object (object 0).
-template <int PREC, bool SINGLE>
-__device__ __forceinline__ float eval_min(const SceneDev& s, const ObjDev* objs, uint32_t ob,
-                                          uint32_t oe, float qx, float qy, float qz, float& best_un,
-                                          uint32_t& best_i, LaneCache& lc) {
-  if (SINGLE) {
-    best_i = 0;
-    return eval_obj<PREC>(s, objs[0], qx, qy, qz, &best_un, lc);
-  }
-  float best = kMaxFloat;
-  best_un = kMaxFloat;
-  best_i = ob;
-  for (uint32_t oi = ob; oi < oe; ++oi) {
-    float du;
-    const float d = eval_obj<PREC>(s, objs[oi], qx, qy, qz, &du, lc);
-    if (d < best) {
-      best = d;
-      best_un = du;
-      best_i = oi;
-    }
-  }
-  return best;
-}
-
 // Up to n march steps of a ray through positions covered by EMPTY boxes: each
 // sample is empty_value().  The run stops before a step whose sample is below
 // brk or whose t is past tmax (the full step decides those), after the step
@@ -1081,14 +1056,25 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
   }
 }
 
-// The object table into shared memory, a word a thread (a record of some 400
-// bytes a thread cost a block of a small scene as long as a sample).
-__device__ __forceinline__ void load_objs(ObjDev* sh, const SceneDev& s) {
+// The object table as the point and occlusion kernels read it.  SHARED: up to
+// kMaxObjectsShared records, copied to shared memory a word a thread (a record of
+// 248 bytes a thread cost a block of a small scene as long as a sample); else the
+// device table.
+template <bool SHARED>
+__device__ __forceinline__ void load_objs(ObjSample* sh, const SceneDev& s) {
+  if (!SHARED) return;
+  constexpr uint32_t kWords = sizeof(ObjSample) / 4, kStride = sizeof(ObjDev) / 4;
+  static_assert(sizeof(ObjSample) % 4 == 0 && sizeof(ObjDev) % 4 == 0, "whole words");
   const uint32_t* src = reinterpret_cast<const uint32_t*>(s.objs);
   uint32_t* dst = reinterpret_cast<uint32_t*>(sh);
-  static_assert(sizeof(ObjDev) % 4 == 0, "whole words");
-  for (uint32_t i = threadIdx.x; i < s.n_objs * static_cast<uint32_t>(sizeof(ObjDev) / 4); i += blockDim.x)
-    dst[i] = __ldg(src + i);
+  for (uint32_t i = threadIdx.x; i < s.n_objs * kWords; i += blockDim.x)
+    dst[i] = __ldg(src + i / kWords * kStride + i % kWords);
+  __syncthreads();
+}
+template <bool SHARED>
+__device__ __forceinline__ const ObjSample& obj_at(const ObjSample* sh, const SceneDev& s, uint32_t i) {
+  if (SHARED) return sh[i];
+  return s.objs[i];
 }
 
 constexpr uint32_t kPointLanes = 8;
@@ -1102,12 +1088,11 @@ constexpr uint32_t kAoLanes = 4;  // one per tap
 // bound by instruction fetch and by that chain, 54 us for 300 points near
 // surfaces (20 so) and, as a call, 72 us for 65,536 over the 1.1M-brick scene (56
 // so; there the bound is the samples' loads).
-template <int PREC>
+template <int PREC, bool SHARED>
 __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* __restrict__ pts, uint32_t n,
                                                      float* dist, float* grad, uint16_t* material) {
-  extern __shared__ ObjDev sh_objs[];
-  load_objs(sh_objs, s);
-  __syncthreads();
+  extern __shared__ ObjSample sh_objs[];
+  load_objs<SHARED>(sh_objs, s);
   const uint32_t id = blockIdx.x * (blockDim.x / kPointLanes) + threadIdx.x / kPointLanes;
   const uint32_t j = threadIdx.x % kPointLanes;
   const uint32_t i = min(id, n - 1);  // (every lane takes part in the exchange)
@@ -1137,7 +1122,7 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
     const bool tap = r == rounds || (s.n_objs == 1u && diff);
     const uint32_t ob = tap ? bi : r * kPointLanes + (j + 2u) % kPointLanes;
     if (tap ? !diff : ob >= s.n_objs) continue;
-    const ObjDev& o = sh_objs[ob];
+    const ObjSample& o = obj_at<SHARED>(sh_objs, s, ob);
     float x = px, y = py, z = pz, lx, ly, lz, du;
     // voxelized: central differences of the sampler, eps = 2 voxels, in the
     // object's frame; else of the object, eps = 10 * hit_threshold(0.001)
@@ -1179,7 +1164,7 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
     if (!material) return;
     uint32_t m = 0;
     if (s.n_objs) {
-      const ObjDev& o = sh_objs[bi];
+      const ObjSample& o = obj_at<SHARED>(sh_objs, s, bi);
       if (o.sdf_type == RKF_SDF_ANALYTICAL || best_un < o.vs16) m = material_at(s, o, px, py, pz, lc);
     }
     material[i] = static_cast<uint16_t>(m);
@@ -1189,7 +1174,7 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
   if (!grad) return;
   float nx = 0.0f, ny = 1.0f, nz = 0.0f;
   if (s.n_objs) {
-    const ObjDev& o = sh_objs[bi];
+    const ObjSample& o = obj_at<SHARED>(sh_objs, s, bi);
     const bool vox = o.sdf_type == RKF_SDF_VOXELIZED;
     float wx = g0, wy = g1, wz = g2;
     if (vox) {
@@ -1222,13 +1207,12 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
 // 32 m scene, 64 / 30,000 / 200,003 / 500,000 points: 32 / 35 / 58 / 86 us for a
 // thread per point, 19 / 21 / 44 / 81 us so; 12 blocks an SM (40 registers), as
 // 10 take 46 and 85 for the last two.
-template <int PREC>
+template <int PREC, bool SHARED>
 __global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __restrict__ pos,
                                                    const float* __restrict__ nrm, uint32_t n,
                                                    float* __restrict__ ao) {
-  extern __shared__ ObjDev sh_objs[];
-  load_objs(sh_objs, s);
-  __syncthreads();
+  extern __shared__ ObjSample sh_objs[];
+  load_objs<SHARED>(sh_objs, s);
   const uint64_t id = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kAoLanes;
   const uint32_t k = 1u + threadIdx.x % kAoLanes;
   const uint32_t i = id < n ? static_cast<uint32_t>(id) : n - 1u;  // (every lane takes part in the exchange)
@@ -1237,11 +1221,14 @@ __global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __r
   const float px = pos[i3], py = pos[i3 + 1], pz = pos[i3 + 2];
   const float nx = nrm[i3], ny = nrm[i3 + 1], nz = nrm[i3 + 2];
   const float dist = __fmul_rn(0.12f, static_cast<float>(k));
-  float du;
-  uint32_t bi;
-  const float d = eval_min<PREC, false>(s, sh_objs, 0, s.n_objs, __fadd_rn(px, __fmul_rn(nx, dist)),
-                                       __fadd_rn(py, __fmul_rn(ny, dist)), __fadd_rn(pz, __fmul_rn(nz, dist)), du,
-                                       bi, lc);
+  const float qx = __fadd_rn(px, __fmul_rn(nx, dist)), qy = __fadd_rn(py, __fmul_rn(ny, dist)),
+              qz = __fadd_rn(pz, __fmul_rn(nz, dist));
+  float d = kMaxFloat;
+  for (uint32_t oi = 0; oi < s.n_objs; ++oi) {
+    float du;
+    const float v = eval_obj<PREC>(s, obj_at<SHARED>(sh_objs, s, oi), qx, qy, qz, &du, lc);
+    if (v < d) d = v;
+  }
   const float tap = __fsub_rn(dist, d);
   float acc = 0.0f, scale = 1.0f;
 #pragma unroll
@@ -1862,20 +1849,34 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
   return c->march_event(st, true);
 }
 
+namespace {
+template <int PREC>
+void query_points(const SceneDev& s, const float* pts, uint32_t n, float* d, float* g, uint16_t* m, cudaStream_t st) {
+  const unsigned blocks = (n - 1) / (128 / detail::kPointLanes) + 1;
+  if (s.n_objs <= kMaxObjectsShared)
+    detail::k_query_points<PREC, true><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, pts, n, d, g, m);
+  else
+    detail::k_query_points<PREC, false><<<blocks, 128, 0, st>>>(s, pts, n, d, g, m);
+}
+
+template <int PREC>
+void sdf_ao(const SceneDev& s, const float* pos, const float* nrm, uint32_t n, float* ao, cudaStream_t st) {
+  const unsigned blocks = (n - 1) / (128 / detail::kAoLanes) + 1;
+  if (s.n_objs <= kMaxObjectsShared)
+    detail::k_sdf_ao<PREC, true><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, pos, nrm, n, ao);
+  else
+    detail::k_sdf_ao<PREC, false><<<blocks, 128, 0, st>>>(s, pos, nrm, n, ao);
+}
+}  // namespace
+
 rkf_status launch_query(Ctx* c, const float* pts, uint32_t n, float* d, float* g, uint16_t* m,
                         cudaStream_t st) {
   if (n == 0) return RKF_OK;
-  const size_t smem = sizeof(ObjDev) * std::max<uint32_t>(1, c->obj_count());
-  const unsigned blocks = (n - 1) / (128 / detail::kPointLanes) + 1;
+  const SceneDev s = c->scene_dev();
   switch (c->cfg.precision) {
-    case RKF_PRECISION_F32:
-      detail::k_query_points<RKF_PRECISION_F32><<<blocks, 128, smem, st>>>(c->scene_dev(), pts, n, d, g, m);
-      break;
-    case RKF_PRECISION_U8:
-      detail::k_query_points<RKF_PRECISION_U8><<<blocks, 128, smem, st>>>(c->scene_dev(), pts, n, d, g, m);
-      break;
-    default:
-      detail::k_query_points<RKF_PRECISION_F16><<<blocks, 128, smem, st>>>(c->scene_dev(), pts, n, d, g, m);
+    case RKF_PRECISION_F32: query_points<RKF_PRECISION_F32>(s, pts, n, d, g, m, st); break;
+    case RKF_PRECISION_U8: query_points<RKF_PRECISION_U8>(s, pts, n, d, g, m, st); break;
+    default: query_points<RKF_PRECISION_F16>(s, pts, n, d, g, m, st);
   }
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());
@@ -1884,17 +1885,11 @@ rkf_status launch_query(Ctx* c, const float* pts, uint32_t n, float* d, float* g
 
 rkf_status launch_ao(Ctx* c, const float* pos, const float* nrm, uint32_t n, float* ao, cudaStream_t st) {
   if (n == 0) return RKF_OK;
-  const size_t smem = sizeof(ObjDev) * std::max<uint32_t>(1, c->obj_count());
-  const unsigned blocks = (n - 1) / (128 / detail::kAoLanes) + 1;
+  const SceneDev s = c->scene_dev();
   switch (c->cfg.precision) {
-    case RKF_PRECISION_F32:
-      detail::k_sdf_ao<RKF_PRECISION_F32><<<blocks, 128, smem, st>>>(c->scene_dev(), pos, nrm, n, ao);
-      break;
-    case RKF_PRECISION_U8:
-      detail::k_sdf_ao<RKF_PRECISION_U8><<<blocks, 128, smem, st>>>(c->scene_dev(), pos, nrm, n, ao);
-      break;
-    default:
-      detail::k_sdf_ao<RKF_PRECISION_F16><<<blocks, 128, smem, st>>>(c->scene_dev(), pos, nrm, n, ao);
+    case RKF_PRECISION_F32: sdf_ao<RKF_PRECISION_F32>(s, pos, nrm, n, ao, st); break;
+    case RKF_PRECISION_U8: sdf_ao<RKF_PRECISION_U8>(s, pos, nrm, n, ao, st); break;
+    default: sdf_ao<RKF_PRECISION_F16>(s, pos, nrm, n, ao, st);
   }
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());

@@ -30,7 +30,7 @@ struct PlainParams {
   float* motion;
 };
 
-__device__ __forceinline__ uint32_t plain_lookup(const PlainParams& kp, const ObjDev& o, uint32_t bx,
+__device__ __forceinline__ uint32_t plain_lookup(const PlainParams& kp, const ObjSample& o, uint32_t bx,
                                                  uint32_t by, uint32_t bz) {
   if (o.has_flat)
     return kp.s.flat_maps[static_cast<size_t>(o.map_off) + bx + static_cast<size_t>(by) * o.bdims[0] +
@@ -39,7 +39,7 @@ __device__ __forceinline__ uint32_t plain_lookup(const PlainParams& kp, const Ob
 }
 
 // sample_voxel_at / sample_voxel_at_grad (ray_march.wgsl:270-315)
-__device__ __forceinline__ float plain_voxel(const PlainParams& kp, const ObjDev& o, int vx, int vy,
+__device__ __forceinline__ float plain_voxel(const PlainParams& kp, const ObjSample& o, int vx, int vy,
                                              int vz, bool grad) {
   const int cx = clampi(vx, 0, o.tv[0] - 1), cy = clampi(vy, 0, o.tv[1] - 1),
             cz = clampi(vz, 0, o.tv[2] - 1);
@@ -51,7 +51,7 @@ __device__ __forceinline__ float plain_voxel(const PlainParams& kp, const ObjDev
 }
 
 // sample_voxelized / sample_voxelized_grad (ray_march.wgsl:353-498)
-__device__ float plain_sample(const PlainParams& kp, const ObjDev& o, float lx, float ly, float lz,
+__device__ float plain_sample(const PlainParams& kp, const ObjSample& o, float lx, float ly, float lz,
                               bool grad) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]), gpy = __fadd_rn(ly, o.half_gs[1]),
               gpz = __fadd_rn(lz, o.half_gs[2]);
@@ -87,7 +87,7 @@ __device__ float plain_sample(const PlainParams& kp, const ObjDev& o, float lx, 
 }
 
 // nearest voxel (ray_march.wgsl:540-596); returns slot or sentinel
-__device__ uint32_t plain_nearest(const PlainParams& kp, const ObjDev& o, float lx, float ly, float lz,
+__device__ uint32_t plain_nearest(const PlainParams& kp, const ObjSample& o, float lx, float ly, float lz,
                                   size_t* vi) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]), gpy = __fadd_rn(ly, o.half_gs[1]),
               gpz = __fadd_rn(lz, o.half_gs[2]);
@@ -102,7 +102,7 @@ __device__ uint32_t plain_nearest(const PlainParams& kp, const ObjDev& o, float 
 }
 
 // evaluate_object (ray_march.wgsl:600-634) with the eager material read
-__device__ float plain_eval(const PlainParams& kp, const ObjDev& o, float wx, float wy, float wz,
+__device__ float plain_eval(const PlainParams& kp, const ObjSample& o, float wx, float wy, float wz,
                             uint32_t* mat) {
   if (o.sdf_type == RKF_SDF_NONE) {
     *mat = 0;
@@ -127,7 +127,7 @@ __device__ float plain_eval(const PlainParams& kp, const ObjDev& o, float wx, fl
 }
 
 __global__ void __launch_bounds__(64) k_march_plain(PlainParams kp) {
-  extern __shared__ ObjDev objs[];
+  extern __shared__ ObjSample objs[];
   const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
   for (uint32_t i = tid; i < kp.s.n_objs; i += blockDim.x * blockDim.y) objs[i] = kp.s.objs[i];
   __syncthreads();
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(64) k_march_plain(PlainParams kp) {
   if (hit) {
     flags |= RKF_FLAG_HIT;
     if (bisected) flags |= RKF_FLAG_BISECTED;
-    const ObjDev& o = objs[robj];
+    const ObjSample& o = objs[robj];
     hx = __fadd_rn(ox, __fmul_rn(dx, rt));
     hy = __fadd_rn(oy, __fmul_rn(dy, rt));
     hz = __fadd_rn(oz, __fmul_rn(dz, rt));
@@ -294,7 +294,7 @@ struct PlainRays {
 // One thread per ray: the same reference loop for generic ray casts
 // (closest hit, any hit, soft shadow of shade_common_shading.wgsl:9-33).
 __global__ void __launch_bounds__(128) k_trace_plain(PlainRays r) {
-  extern __shared__ ObjDev objs[];
+  extern __shared__ ObjSample objs[];
   for (uint32_t i = threadIdx.x; i < r.kp.s.n_objs; i += blockDim.x) objs[i] = r.kp.s.objs[i];
   __syncthreads();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(128) k_trace_plain(PlainRays r) {
   float nxo = 0, nyo = 0, nzo = 0;
   uint32_t slot = RKF_EMPTY_SLOT;
   if (hit) {
-    const ObjDev& o = objs[robj];
+    const ObjSample& o = objs[robj];
     const float hx = __fadd_rn(ox, __fmul_rn(dx, rt)), hy = __fadd_rn(oy, __fmul_rn(dy, rt)),
                 hz = __fadd_rn(oz, __fmul_rn(dz, rt));
     if (o.sdf_type == RKF_SDF_VOXELIZED) {
@@ -469,7 +469,7 @@ rkf_status launch_trace_plain(Ctx* c, const float* o, const float* d, const floa
   r.tmax = tmax;
   r.n = n;
   r.mode = mode;
-  const size_t smem = sizeof(ObjDev) * (c->obj_count() ? c->obj_count() : 1);
+  const size_t smem = sizeof(ObjSample) * (c->obj_count() ? c->obj_count() : 1);
   detail::k_trace_plain<<<(n + 127) / 128, 128, smem, st>>>(r);
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());
@@ -506,7 +506,7 @@ rkf_status launch_plain(Ctx* c, const rkf_camera* cam, const rkf_march_params* p
   kp.motion = out.motion;
   const dim3 block(8, 8);
   const dim3 grid((w + 7) / 8, (h + 7) / 8);
-  const size_t smem = sizeof(ObjDev) * (c->obj_count() ? c->obj_count() : 1);
+  const size_t smem = sizeof(ObjSample) * (c->obj_count() ? c->obj_count() : 1);
   detail::k_march_plain<<<grid, block, smem, st>>>(kp);
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());

@@ -35,7 +35,7 @@ __device__ __forceinline__ float mix3_const(float c, float tx, float ty, float t
 }
 
 template <int PREC>
-__device__ __forceinline__ float corner(const SceneDev& s, const ObjDev& o, uint32_t slot,
+__device__ __forceinline__ float corner(const SceneDev& s, const ObjSample& o, uint32_t slot,
                                         uint32_t idx, bool grad) {
   if (slot == RKF_EMPTY_SLOT) return o.be;                      // vs * 8
   if (slot == RKF_INTERIOR_SLOT) return grad ? -o.be : -o.vs2;  // -(vs*8) / -(vs*2)
@@ -51,7 +51,7 @@ __device__ __forceinline__ uint32_t resolve_top(const SceneDev& s, uint32_t blk,
 }
 
 // slot of brick (bx,by,bz) (or a sentinel) through the memo
-__device__ __forceinline__ uint32_t lookup_cached(const SceneDev& s, const ObjDev& o, uint32_t bx,
+__device__ __forceinline__ uint32_t lookup_cached(const SceneDev& s, const ObjSample& o, uint32_t bx,
                                                   uint32_t by, uint32_t bz, LaneCache& lc) {
   const uint32_t tv = resolve_top(s, top_index(o, bx, by, bz), lc);
   if (tv >= RKF_INTERIOR_SLOT) return tv;
@@ -69,7 +69,7 @@ __device__ __forceinline__ uint32_t lookup_cached(const SceneDev& s, const ObjDe
 // neither the IEEE quotient nor the wide floor: less code, and the march is
 // bound by fetching its code.
 template <int PREC, bool SIMPLE = false>
-__device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, float lx, float ly,
+__device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjSample& o, float lx, float ly,
                                             float lz, bool grad, LaneCache& lc) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]);
   const float gpy = __fadd_rn(ly, o.half_gs[1]);
@@ -227,7 +227,7 @@ __device__ __forceinline__ float sample_vox(const SceneDev& s, const ObjDev& o, 
 
 // Nearest-voxel slot lookup of sample_voxelized_material / _blend_data.  (Out
 // of line, as everything that only hits need: see sample_vox.)
-static __device__ __noinline__ uint32_t nearest_slot(const SceneDev& s, const ObjDev& o, float lx,
+static __device__ __noinline__ uint32_t nearest_slot(const SceneDev& s, const ObjSample& o, float lx,
                                                  float ly, float lz, uint32_t& idx, LaneCache& lc) {
   const float gpx = __fadd_rn(lx, o.half_gs[0]);
   const float gpy = __fadd_rn(ly, o.half_gs[1]);
@@ -245,7 +245,7 @@ static __device__ __noinline__ uint32_t nearest_slot(const SceneDev& s, const Ob
 // equals x up to the sign of a zero, and every consumer of the local
 // coordinate adds a nonzero offset to it or compares it, so x + m12 gives the
 // same downstream bits as the full product.
-__device__ __forceinline__ void to_local_fast(const ObjDev& o, float wx, float wy, float wz,
+__device__ __forceinline__ void to_local_fast(const ObjSample& o, float wx, float wy, float wz,
                                               float& lx, float& ly, float& lz) {
   if (o.translate_only) {
     lx = __fadd_rn(wx, o.m[12]);
@@ -260,7 +260,7 @@ __device__ __forceinline__ void to_local_fast(const ObjDev& o, float wx, float w
 // *unscaled receives the sampler's value (the material-lookup test of
 // ray_march.wgsl:621 compares it with vs*16).
 template <int PREC>
-__device__ __forceinline__ float eval_obj(const SceneDev& s, const ObjDev& o, float wx, float wy,
+__device__ __forceinline__ float eval_obj(const SceneDev& s, const ObjSample& o, float wx, float wy,
                                           float wz, float* unscaled, LaneCache& lc) {
   if (o.sdf_type == RKF_SDF_NONE) {
     *unscaled = kMaxFloat;
@@ -276,7 +276,7 @@ __device__ __forceinline__ float eval_obj(const SceneDev& s, const ObjDev& o, fl
 
 // Material evaluate_object would report at world position w for object o
 // (ray_march.wgsl:613-626).
-__device__ __forceinline__ uint32_t material_at(const SceneDev& s, const ObjDev& o, float wx,
+__device__ __forceinline__ uint32_t material_at(const SceneDev& s, const ObjSample& o, float wx,
                                                 float wy, float wz, LaneCache& lc) {
   if (o.sdf_type == RKF_SDF_ANALYTICAL) return o.material_id;
   if (o.sdf_type != RKF_SDF_VOXELIZED) return 0u;
