@@ -1056,13 +1056,20 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
   }
 }
 
-// The object table as the point and occlusion kernels read it.  SHARED: up to
-// kMaxObjectsShared records, copied to shared memory a word a thread (a record of
-// 248 bytes a thread cost a block of a small scene as long as a sample); else the
-// device table.
-template <bool SHARED>
-__device__ __forceinline__ void load_objs(ObjSample* sh, const SceneDev& s) {
-  if (!SHARED) return;
+// Where a kernel reads the object table: the launch parameters (a scene of one
+// object), a copy in shared memory (up to kMaxObjectsShared records, a word a
+// thread: a record a thread cost a block of a small scene as long as a sample), or
+// the device table.
+enum : int { TABLE_ONE = 0, TABLE_SHARED = 1, TABLE_DEVICE = 2 };
+template <int TABLE>
+struct TableArg {};
+template <>
+struct TableArg<TABLE_ONE> {
+  ObjSample one;
+};
+template <int TABLE>
+__device__ __forceinline__ void load_table(ObjSample* sh, const SceneDev& s) {
+  if (TABLE != TABLE_SHARED) return;
   constexpr uint32_t kWords = sizeof(ObjSample) / 4, kStride = sizeof(ObjDev) / 4;
   static_assert(sizeof(ObjSample) % 4 == 0 && sizeof(ObjDev) % 4 == 0, "whole words");
   const uint32_t* src = reinterpret_cast<const uint32_t*>(s.objs);
@@ -1070,11 +1077,6 @@ __device__ __forceinline__ void load_objs(ObjSample* sh, const SceneDev& s) {
   for (uint32_t i = threadIdx.x; i < s.n_objs * kWords; i += blockDim.x)
     dst[i] = __ldg(src + i / kWords * kStride + i % kWords);
   __syncthreads();
-}
-template <bool SHARED>
-__device__ __forceinline__ const ObjSample& obj_at(const ObjSample* sh, const SceneDev& s, uint32_t i) {
-  if (SHARED) return sh[i];
-  return s.objs[i];
 }
 
 constexpr uint32_t kPointLanes = 8;
@@ -1088,11 +1090,26 @@ constexpr uint32_t kAoLanes = 4;  // one per tap
 // bound by instruction fetch and by that chain, 54 us for 300 points near
 // surfaces (20 so) and, as a call, 72 us for 65,536 over the 1.1M-brick scene (56
 // so; there the bound is the samples' loads).
-template <int PREC, bool SHARED>
-__global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* __restrict__ pts, uint32_t n,
-                                                     float* dist, float* grad, uint16_t* material) {
+// A block serves 16 points, and with more than kPointFewObjects objects a copy of
+// the table for these costs more than reading the device table, which the
+// first-level cache holds: 65,536 points, 60 / 100 / 163 / 198 objects: 80 / 98 / 120 /
+// 133 us so, 89 / 123 / 226 / 282 with the copy (a thread per point, 128 to a copy: 97 /
+// 115 / 139 / 144); 2 / 5 / 8 / 12 / 24 objects: 56.2 / 57.2 / 57.1 / 60.3 / 63.8
+// against 53.9 / 56.0 / 56.3 / 60.3 / 65.9.  One object from the launch parameters:
+// 49 us for the 65,536 over the 1.1M-brick scene, 57 with the copy.
+constexpr uint32_t kPointFewObjects = 12;
+template <int PREC, int TABLE>
+__global__ void __launch_bounds__(128) k_query_points(SceneDev s, const __grid_constant__ TableArg<TABLE> arg,
+                                                     const float* __restrict__ pts, uint32_t n, float* dist,
+                                                     float* grad, uint16_t* material) {
   extern __shared__ ObjSample sh_objs[];
-  load_objs<SHARED>(sh_objs, s);
+  load_table<TABLE>(sh_objs, s);
+  const ObjDev* const table = s.objs;
+  const auto object = [&](uint32_t k) -> const ObjSample& {
+    if constexpr (TABLE == TABLE_ONE) return arg.one;
+    else if constexpr (TABLE == TABLE_SHARED) return sh_objs[k];
+    else return table[k];
+  };
   const uint32_t id = blockIdx.x * (blockDim.x / kPointLanes) + threadIdx.x / kPointLanes;
   const uint32_t j = threadIdx.x % kPointLanes;
   const uint32_t i = min(id, n - 1);  // (every lane takes part in the exchange)
@@ -1102,7 +1119,8 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
   float best = kMaxFloat, best_un = kMaxFloat, g = 0.0f;
   uint32_t bi = 0;
   const bool diff = grad != nullptr && j < 6u;
-  const uint32_t rounds = (s.n_objs + kPointLanes - 1u) / kPointLanes;
+  const uint32_t n_objs = TABLE == TABLE_ONE ? 1u : s.n_objs;
+  const uint32_t rounds = (n_objs + kPointLanes - 1u) / kPointLanes;
 #pragma unroll 1
   for (uint32_t r = 0; r <= rounds; ++r) {
     if (r == rounds) {
@@ -1117,12 +1135,12 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
           bi = b2;
         }
       }
-      if (s.n_objs <= 1u || !grad) break;
+      if (n_objs <= 1u || !grad) break;
     }
-    const bool tap = r == rounds || (s.n_objs == 1u && diff);
+    const bool tap = r == rounds || (n_objs == 1u && diff);
     const uint32_t ob = tap ? bi : r * kPointLanes + (j + 2u) % kPointLanes;
-    if (tap ? !diff : ob >= s.n_objs) continue;
-    const ObjSample& o = obj_at<SHARED>(sh_objs, s, ob);
+    if (tap ? !diff : ob >= n_objs) continue;
+    const ObjSample& o = object(ob);
     float x = px, y = py, z = pz, lx, ly, lz, du;
     // voxelized: central differences of the sampler, eps = 2 voxels, in the
     // object's frame; else of the object, eps = 10 * hit_threshold(0.001)
@@ -1163,8 +1181,8 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
   if (j == 7u) {
     if (!material) return;
     uint32_t m = 0;
-    if (s.n_objs) {
-      const ObjSample& o = obj_at<SHARED>(sh_objs, s, bi);
+    if (n_objs) {
+      const ObjSample& o = object(bi);
       if (o.sdf_type == RKF_SDF_ANALYTICAL || best_un < o.vs16) m = material_at(s, o, px, py, pz, lc);
     }
     material[i] = static_cast<uint16_t>(m);
@@ -1173,8 +1191,8 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
   if (dist) dist[i] = best;
   if (!grad) return;
   float nx = 0.0f, ny = 1.0f, nz = 0.0f;
-  if (s.n_objs) {
-    const ObjSample& o = obj_at<SHARED>(sh_objs, s, bi);
+  if (n_objs) {
+    const ObjSample& o = object(bi);
     const bool vox = o.sdf_type == RKF_SDF_VOXELIZED;
     float wx = g0, wy = g1, wz = g2;
     if (vox) {
@@ -1207,37 +1225,44 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const float* _
 // 32 m scene, 64 / 30,000 / 200,003 / 500,000 points: 32 / 35 / 58 / 86 us for a
 // thread per point, 19 / 21 / 44 / 81 us so; 12 blocks an SM (40 registers), as
 // 10 take 46 and 85 for the last two.
-template <int PREC, bool SHARED>
+// Every lane of a warp evaluates the same object, from a copy of the table where it
+// fits.  A block takes its points in turns, so that a launch copies the table for
+// the blocks that fit the chip alone (ao_blocks).
+template <int PREC, int TABLE>
 __global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __restrict__ pos,
                                                    const float* __restrict__ nrm, uint32_t n,
                                                    float* __restrict__ ao) {
   extern __shared__ ObjSample sh_objs[];
-  load_objs<SHARED>(sh_objs, s);
-  const uint64_t id = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kAoLanes;
-  const uint32_t k = 1u + threadIdx.x % kAoLanes;
-  const uint32_t i = id < n ? static_cast<uint32_t>(id) : n - 1u;  // (every lane takes part in the exchange)
-  LaneCache lc;
-  const size_t i3 = 3 * static_cast<size_t>(i);
-  const float px = pos[i3], py = pos[i3 + 1], pz = pos[i3 + 2];
-  const float nx = nrm[i3], ny = nrm[i3 + 1], nz = nrm[i3 + 2];
-  const float dist = __fmul_rn(0.12f, static_cast<float>(k));
-  const float qx = __fadd_rn(px, __fmul_rn(nx, dist)), qy = __fadd_rn(py, __fmul_rn(ny, dist)),
-              qz = __fadd_rn(pz, __fmul_rn(nz, dist));
-  float d = kMaxFloat;
-  for (uint32_t oi = 0; oi < s.n_objs; ++oi) {
-    float du;
-    const float v = eval_obj<PREC>(s, obj_at<SHARED>(sh_objs, s, oi), qx, qy, qz, &du, lc);
-    if (v < d) d = v;
-  }
-  const float tap = __fsub_rn(dist, d);
-  float acc = 0.0f, scale = 1.0f;
+  load_table<TABLE>(sh_objs, s);
+  const uint32_t k = 1u + threadIdx.x % kAoLanes, per = blockDim.x / kAoLanes;
+#pragma unroll 1
+  for (uint64_t first = static_cast<uint64_t>(blockIdx.x) * per; first < n; first += static_cast<uint64_t>(gridDim.x) * per) {
+    const uint64_t id = first + threadIdx.x / kAoLanes;
+    const uint32_t i = id < n ? static_cast<uint32_t>(id) : n - 1u;  // (every lane takes part in the exchange)
+    LaneCache lc;
+    const size_t i3 = 3 * static_cast<size_t>(i);
+    const float px = pos[i3], py = pos[i3 + 1], pz = pos[i3 + 2];
+    const float nx = nrm[i3], ny = nrm[i3 + 1], nz = nrm[i3 + 2];
+    const float dist = __fmul_rn(0.12f, static_cast<float>(k));
+    const float qx = __fadd_rn(px, __fmul_rn(nx, dist)), qy = __fadd_rn(py, __fmul_rn(ny, dist)),
+                qz = __fadd_rn(pz, __fmul_rn(nz, dist));
+    float d = kMaxFloat;
+    for (uint32_t oi = 0; oi < s.n_objs; ++oi) {
+      const ObjSample* o = s.objs + oi;
+      if (TABLE == TABLE_SHARED) o = sh_objs + oi;
+      float du;
+      const float v = eval_obj<PREC>(s, *o, qx, qy, qz, &du, lc);
+      if (v < d) d = v;
+    }
+    const float tap = __fsub_rn(dist, d);
+    float acc = 0.0f, scale = 1.0f;
 #pragma unroll
-  for (int a = 0; a < static_cast<int>(kAoLanes); ++a) {  // in the taps' order
-    acc = __fadd_rn(acc, __fmul_rn(scale, __shfl_sync(kFull, tap, a, kAoLanes)));
-    scale = __fmul_rn(scale, 0.5f);
+    for (int a = 0; a < static_cast<int>(kAoLanes); ++a) {  // in the taps' order
+      acc = __fadd_rn(acc, __fmul_rn(scale, __shfl_sync(kFull, tap, a, kAoLanes)));
+      scale = __fmul_rn(scale, 0.5f);
+    }
+    if (id < n && k == 1u) ao[i] = clampf(__fsub_rn(1.0f, __fmul_rn(0.7f, acc)), 0.0f, 1.0f);
   }
-  if (id >= n || k != 1u) return;
-  ao[i] = clampf(__fsub_rn(1.0f, __fmul_rn(0.7f, acc)), 0.0f, 1.0f);
 }
 
 template <int PREC>
@@ -1851,32 +1876,48 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
 
 namespace {
 template <int PREC>
-void query_points(const SceneDev& s, const float* pts, uint32_t n, float* d, float* g, uint16_t* m, cudaStream_t st) {
-  const unsigned blocks = (n - 1) / (128 / detail::kPointLanes) + 1;
-  if (s.n_objs <= kMaxObjectsShared)
-    detail::k_query_points<PREC, true><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, pts, n, d, g, m);
+void query_points(const Ctx* c, const float* pts, uint32_t n, float* d, float* g, uint16_t* m, cudaStream_t st) {
+  using namespace detail;
+  const SceneDev s = c->scene_dev();
+  const unsigned blocks = (n - 1) / (128 / kPointLanes) + 1;
+  if (s.n_objs == 1)
+    k_query_points<PREC, TABLE_ONE><<<blocks, 128, 0, st>>>(s, {c->objdev_host[0]}, pts, n, d, g, m);
+  else if (s.n_objs <= kPointFewObjects)
+    k_query_points<PREC, TABLE_SHARED><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, {}, pts, n, d, g, m);
   else
-    detail::k_query_points<PREC, false><<<blocks, 128, 0, st>>>(s, pts, n, d, g, m);
+    k_query_points<PREC, TABLE_DEVICE><<<blocks, 128, 0, st>>>(s, {}, pts, n, d, g, m);
+}
+
+// Blocks of an occlusion launch: one for every 32 of its points or, where they copy
+// the table and it holds more than kAoFewObjects objects, those that fit the chip (65,536 points, 16 / 32 / 60 / 163 /
+// 198 objects: 39 / 49 / 68 / 177 / 257 us for a block per 32 points, 39 / 47 / 62 /
+// 152 / 209 so; 1 and 5 objects: 27.6 and 32.4 against 29.3 and 33.2).
+constexpr uint32_t kAoFewObjects = 16;
+unsigned ao_blocks(const Ctx* c, uint32_t n, uint32_t n_objs) {
+  const unsigned all = (n - 1) / (128 / detail::kAoLanes) + 1;
+  if (n_objs <= kAoFewObjects || n_objs > kMaxObjectsShared) return all;
+  const unsigned fit = static_cast<unsigned>((227u << 10) / (sizeof(ObjSample) * n_objs + 1024u));
+  return std::min(all, static_cast<unsigned>(c->sm_count) * std::max(1u, std::min(12u, fit)));
 }
 
 template <int PREC>
-void sdf_ao(const SceneDev& s, const float* pos, const float* nrm, uint32_t n, float* ao, cudaStream_t st) {
-  const unsigned blocks = (n - 1) / (128 / detail::kAoLanes) + 1;
+void sdf_ao(const Ctx* c, const SceneDev& s, const float* pos, const float* nrm, uint32_t n, float* ao,
+            cudaStream_t st) {
+  const unsigned blocks = ao_blocks(c, n, s.n_objs);
   if (s.n_objs <= kMaxObjectsShared)
-    detail::k_sdf_ao<PREC, true><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, pos, nrm, n, ao);
+    detail::k_sdf_ao<PREC, detail::TABLE_SHARED><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, pos, nrm, n, ao);
   else
-    detail::k_sdf_ao<PREC, false><<<blocks, 128, 0, st>>>(s, pos, nrm, n, ao);
+    detail::k_sdf_ao<PREC, detail::TABLE_DEVICE><<<blocks, 128, 0, st>>>(s, pos, nrm, n, ao);
 }
 }  // namespace
 
 rkf_status launch_query(Ctx* c, const float* pts, uint32_t n, float* d, float* g, uint16_t* m,
                         cudaStream_t st) {
   if (n == 0) return RKF_OK;
-  const SceneDev s = c->scene_dev();
   switch (c->cfg.precision) {
-    case RKF_PRECISION_F32: query_points<RKF_PRECISION_F32>(s, pts, n, d, g, m, st); break;
-    case RKF_PRECISION_U8: query_points<RKF_PRECISION_U8>(s, pts, n, d, g, m, st); break;
-    default: query_points<RKF_PRECISION_F16>(s, pts, n, d, g, m, st);
+    case RKF_PRECISION_F32: query_points<RKF_PRECISION_F32>(c, pts, n, d, g, m, st); break;
+    case RKF_PRECISION_U8: query_points<RKF_PRECISION_U8>(c, pts, n, d, g, m, st); break;
+    default: query_points<RKF_PRECISION_F16>(c, pts, n, d, g, m, st);
   }
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());
@@ -1887,9 +1928,9 @@ rkf_status launch_ao(Ctx* c, const float* pos, const float* nrm, uint32_t n, flo
   if (n == 0) return RKF_OK;
   const SceneDev s = c->scene_dev();
   switch (c->cfg.precision) {
-    case RKF_PRECISION_F32: sdf_ao<RKF_PRECISION_F32>(s, pos, nrm, n, ao, st); break;
-    case RKF_PRECISION_U8: sdf_ao<RKF_PRECISION_U8>(s, pos, nrm, n, ao, st); break;
-    default: sdf_ao<RKF_PRECISION_F16>(s, pos, nrm, n, ao, st);
+    case RKF_PRECISION_F32: sdf_ao<RKF_PRECISION_F32>(c, s, pos, nrm, n, ao, st); break;
+    case RKF_PRECISION_U8: sdf_ao<RKF_PRECISION_U8>(c, s, pos, nrm, n, ao, st); break;
+    default: sdf_ao<RKF_PRECISION_F16>(c, s, pos, nrm, n, ao, st);
   }
   c->counted();
   RKF_CUDA_TRY(cudaGetLastError());

@@ -11,7 +11,7 @@ from test_tiled_gpu import PLANES, _params
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n_objs", [2, 32, 33, 163, 164, 198, 199, 300])
+@pytest.mark.parametrize("n_objs", [2, 12, 13, 32, 33, 163, 164, 198, 199, 300])
 def test_queries_over_many_objects(oracle, small_scene, n_objs):
     from rkifield_b200 import scenes
     v = small_scene["vox"]
