@@ -1098,7 +1098,7 @@ constexpr uint32_t kAoLanes = 4;  // one per tap
 // against 53.9 / 56.0 / 56.3 / 60.3 / 65.9.  One object from the launch parameters:
 // 49 us for the 65,536 over the 1.1M-brick scene, 57 with the copy.
 constexpr uint32_t kPointFewObjects = 12;
-template <int PREC, int TABLE>
+template <int PREC, int TABLE, uint32_t LANES>
 __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const __grid_constant__ TableArg<TABLE> arg,
                                                      const float* __restrict__ pts, uint32_t n, float* dist,
                                                      float* grad, uint16_t* material) {
@@ -1110,23 +1110,24 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const __grid_c
     else if constexpr (TABLE == TABLE_SHARED) return sh_objs[k];
     else return table[k];
   };
-  const uint32_t id = blockIdx.x * (blockDim.x / kPointLanes) + threadIdx.x / kPointLanes;
-  const uint32_t j = threadIdx.x % kPointLanes;
+  const uint32_t id = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+  const uint32_t j = threadIdx.x % LANES;
   const uint32_t i = min(id, n - 1);  // (every lane takes part in the exchange)
   LaneCache lc;
   const float px = pts[3 * static_cast<size_t>(i)], py = pts[3 * static_cast<size_t>(i) + 1],
               pz = pts[3 * static_cast<size_t>(i) + 2];
   float best = kMaxFloat, best_un = kMaxFloat, g = 0.0f;
   uint32_t bi = 0;
-  const bool diff = grad != nullptr && j < 6u;
+  const bool taps = LANES > 1u && grad != nullptr;  // (a thread per point takes none)
+  const bool diff = taps && j < 6u;
   const uint32_t n_objs = TABLE == TABLE_ONE ? 1u : s.n_objs;
-  const uint32_t rounds = (n_objs + kPointLanes - 1u) / kPointLanes;
+  const uint32_t rounds = (n_objs + LANES - 1u) / LANES;
 #pragma unroll 1
   for (uint32_t r = 0; r <= rounds; ++r) {
     if (r == rounds) {
       // the point's object: the smallest value, the first of equal ones
 #pragma unroll
-      for (int m = kPointLanes / 2; m; m >>= 1) {
+      for (int m = LANES / 2; m; m >>= 1) {
         const float d2 = __shfl_xor_sync(kFull, best, m), u2 = __shfl_xor_sync(kFull, best_un, m);
         const uint32_t b2 = __shfl_xor_sync(kFull, bi, m);
         if (d2 < best || (d2 == best && b2 < bi)) {
@@ -1135,10 +1136,10 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const __grid_c
           bi = b2;
         }
       }
-      if (n_objs <= 1u || !grad) break;
+      if (n_objs <= 1u || !taps) break;
     }
     const bool tap = r == rounds || (n_objs == 1u && diff);
-    const uint32_t ob = tap ? bi : r * kPointLanes + (j + 2u) % kPointLanes;
+    const uint32_t ob = tap ? bi : r * LANES + (j + 2u) % LANES;
     if (tap ? !diff : ob >= n_objs) continue;
     const ObjSample& o = object(ob);
     float x = px, y = py, z = pz, lx, ly, lz, du;
@@ -1173,23 +1174,22 @@ __global__ void __launch_bounds__(128) k_query_points(SceneDev s, const __grid_c
       bi = ob;
     }
   }
-  g = __fsub_rn(g, __shfl_down_sync(kFull, g, 1, kPointLanes));  // lanes 0, 2, 4
-  const float g0 = __shfl_sync(kFull, g, 0, kPointLanes), g1 = __shfl_sync(kFull, g, 2, kPointLanes),
-              g2 = __shfl_sync(kFull, g, 4, kPointLanes);
-  if (j < 6u || id >= n) return;
+  g = __fsub_rn(g, __shfl_down_sync(kFull, g, 1, LANES));  // lanes 0, 2, 4
+  const float g0 = __shfl_sync(kFull, g, 0, LANES), g1 = __shfl_sync(kFull, g, 2, LANES),
+              g2 = __shfl_sync(kFull, g, 4, LANES);
+  if (id >= n) return;
   // lane 6: distance and gradient; lane 7: the material
-  if (j == 7u) {
-    if (!material) return;
+  if (material && (LANES == 1u || j == 7u)) {
     uint32_t m = 0;
     if (n_objs) {
       const ObjSample& o = object(bi);
       if (o.sdf_type == RKF_SDF_ANALYTICAL || best_un < o.vs16) m = material_at(s, o, px, py, pz, lc);
     }
     material[i] = static_cast<uint16_t>(m);
-    return;
   }
+  if (LANES > 1u && j != 6u) return;
   if (dist) dist[i] = best;
-  if (!grad) return;
+  if (!taps) return;
   float nx = 0.0f, ny = 1.0f, nz = 0.0f;
   if (n_objs) {
     const ObjSample& o = object(bi);
@@ -1875,24 +1875,40 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
 }
 
 namespace {
-template <int PREC>
+template <int PREC, uint32_t LANES>
 void query_points(const Ctx* c, const float* pts, uint32_t n, float* d, float* g, uint16_t* m, cudaStream_t st) {
   using namespace detail;
   const SceneDev s = c->scene_dev();
-  const unsigned blocks = (n - 1) / (128 / kPointLanes) + 1;
+  const unsigned blocks = (n - 1) / (128 / LANES) + 1;
   if (s.n_objs == 1)
-    k_query_points<PREC, TABLE_ONE><<<blocks, 128, 0, st>>>(s, {c->objdev_host[0]}, pts, n, d, g, m);
-  else if (s.n_objs <= kPointFewObjects)
-    k_query_points<PREC, TABLE_SHARED><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, {}, pts, n, d, g, m);
+    k_query_points<PREC, TABLE_ONE, LANES><<<blocks, 128, 0, st>>>(s, {c->objdev_host[0]}, pts, n, d, g, m);
+  else if (s.n_objs <= (LANES == 1 ? kMaxObjectsShared : kPointFewObjects))
+    k_query_points<PREC, TABLE_SHARED, LANES><<<blocks, 128, sizeof(ObjSample) * s.n_objs, st>>>(s, {}, pts, n, d, g, m);
   else
-    k_query_points<PREC, TABLE_DEVICE><<<blocks, 128, 0, st>>>(s, {}, pts, n, d, g, m);
+    k_query_points<PREC, TABLE_DEVICE, LANES><<<blocks, 128, 0, st>>>(s, {}, pts, n, d, g, m);
+}
+
+// A query of distances (and materials) alone has one sample a point and object, for
+// which a thread does: eight lanes serve it while they fit the chip.  16,000 /
+// 65,536 / 500,000 points, 1 object: 27.5 / 35 / 97 us for eight lanes, 27 / 28.7 / 40
+// for a thread; 12 objects 29.8 / 42 / 148 against 29.4 / 31 / 53; 24 objects 28.7 /
+// 45.5 / 168 against 32.5 / 34 / 67; 120 objects 42 / 87 / 425 against 58 / 63 / 202.
+constexpr uint32_t kWidePoints = 1u << 14, kWidePointsMany = 1u << 15;
+template <int PREC>
+void query_points(const Ctx* c, const float* pts, uint32_t n, float* d, float* g, uint16_t* m, cudaStream_t st) {
+  const uint32_t n_objs = c->obj_count();
+  if (!g && n >= (n_objs <= detail::kPointFewObjects ? kWidePoints : kWidePointsMany) && n_objs <= kMaxObjectsShared)
+    query_points<PREC, 1>(c, pts, n, d, g, m, st);
+  else
+    query_points<PREC, detail::kPointLanes>(c, pts, n, d, g, m, st);
 }
 
 // Blocks of an occlusion launch: one for every 32 of its points or, where they copy
-// the table and it holds more than kAoFewObjects objects, those that fit the chip (65,536 points, 16 / 32 / 60 / 163 /
-// 198 objects: 39 / 49 / 68 / 177 / 257 us for a block per 32 points, 39 / 47 / 62 /
-// 152 / 209 so; 1 and 5 objects: 27.6 and 32.4 against 29.3 and 33.2).
-constexpr uint32_t kAoFewObjects = 16;
+// the table and it holds more than kAoFewObjects objects, those that fit the chip
+// (65,536 points, 60 / 100 / 163 / 198 objects: 68 / 94 / 177 / 257 us for a block per 32
+// points, 62 / 90 / 152 / 209 so; but 1,000,000 points, 24 / 60 / 163 objects: 268 / 559 /
+// 2,901 against 283 / 564 / 1,645).
+constexpr uint32_t kAoFewObjects = 64;
 unsigned ao_blocks(const Ctx* c, uint32_t n, uint32_t n_objs) {
   const unsigned all = (n - 1) / (128 / detail::kAoLanes) + 1;
   if (n_objs <= kAoFewObjects || n_objs > kMaxObjectsShared) return all;

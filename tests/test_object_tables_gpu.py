@@ -41,3 +41,26 @@ def test_queries_over_many_objects(oracle, small_scene, n_objs):
                 assert_bits_equal(got[k], ref[k], k)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n_objs", [0, 1, 12, 13, 198, 199])
+def test_distances_alone(small_scene, n_objs):
+    """A query without gradients answers as one with them, on both sides of the
+    sizes at which it takes a thread per point."""
+    import ctypes as C
+
+    from rkifield_b200 import _abi as abi
+    objs = ([small_scene["obj"]] if n_objs == 1 else _objects(small_scene, n_objs - 1, seed=3)) if n_objs else []
+    ctx = _context(small_scene, objs)
+    try:
+        pts = np.random.default_rng(n_objs).uniform(-32.0, 32.0, (32769, 3)).astype(np.float32)
+        d_ref, _, m_ref = ctx.query_points(pts)
+        for n in (1, 16383, 16384, 32767, 32768, 32769):
+            for want_d, want_m in ((True, False), (False, True), (True, True)):
+                d, m = np.zeros(n, np.float32), np.zeros(n, np.uint16)
+                abi.check(ctx.lib.rkf_query_points(ctx.h, pts.ctypes.data, n, d.ctypes.data if want_d else None, None,
+                                                   m.ctypes.data if want_m else None, abi.RKF_MEM_HOST), "query")
+                assert_bits_equal(d, d_ref[:n] if want_d else 0 * d, f"{n}: distance")
+                np.testing.assert_array_equal(m, m_ref[:n] if want_m else 0 * m)
+    finally:
+        ctx.close()
