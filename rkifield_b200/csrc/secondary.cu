@@ -52,6 +52,80 @@ struct SecParams {
   unsigned int* hits;
 };
 
+// A pixel's surface point and normal.
+struct SecHit {
+  float x, y, z, nx, ny, nz;
+  bool hit;
+};
+__device__ __forceinline__ SecHit load_hit(const SecParams& k, uint32_t i, bool live) {
+  SecHit h{0, 0, 0, 0, 1, 0, live && (k.flags[i] & RKF_FLAG_HIT) != 0};
+  if (h.hit) {
+    const uint32_t px = i % k.w, py = i / k.w;
+    const float u = (static_cast<float>(px) + 0.5f) / static_cast<float>(k.w);
+    const float v = (static_cast<float>(py) + 0.5f) / static_cast<float>(k.h);
+    float dx = k.fwd[0] + (u * 2.0f - 1.0f) * k.right[0] + (1.0f - v * 2.0f) * k.up[0];
+    float dy = k.fwd[1] + (u * 2.0f - 1.0f) * k.right[1] + (1.0f - v * 2.0f) * k.up[1];
+    float dz = k.fwd[2] + (u * 2.0f - 1.0f) * k.right[2] + (1.0f - v * 2.0f) * k.up[2];
+    const float il = rsqrtf(dx * dx + dy * dy + dz * dz);
+    dx *= il;
+    dy *= il;
+    dz *= il;
+    const float t = k.t[i];
+    h.x = k.pos[0] + dx * t;
+    h.y = k.pos[1] + dy * t;
+    h.z = k.pos[2] + dz * t;
+    h.nx = k.normal[3 * static_cast<size_t>(i)];
+    h.ny = k.normal[3 * static_cast<size_t>(i) + 1];
+    h.nz = k.normal[3 * static_cast<size_t>(i) + 2];
+  }
+  return h;
+}
+
+// The ray to light l.
+__device__ __forceinline__ float shadow_ray(const SecParams& k, const SecHit& h, uint32_t l, float* o, float* d) {
+  const float ox = h.x + h.nx * k.shadow_bias, oy = h.y + h.ny * k.shadow_bias, oz = h.z + h.nz * k.shadow_bias;
+  float dx = k.lights[3 * l] - ox, dy = k.lights[3 * l + 1] - oy, dz = k.lights[3 * l + 2] - oz;
+  const float len = sqrtf(dx * dx + dy * dy + dz * dz);
+  const float il = len > 0.0f ? 1.0f / len : 0.0f;
+  o[0] = ox;
+  o[1] = oy;
+  o[2] = oz;
+  d[0] = dx * il;
+  d[1] = dy * il;
+  d[2] = dz * il;
+  return h.hit ? len : -1.0f;
+}
+
+// Tangent frame of a normal.
+struct SecFrame {
+  float tx, ty, tz, bx, by, bz;
+};
+__device__ __forceinline__ SecFrame frame_of(const SecHit& h) {
+  const float ax = fabsf(h.nx) < 0.9f ? 1.0f : 0.0f, ay = fabsf(h.nx) < 0.9f ? 0.0f : 1.0f;
+  float tx = ay * h.nz, ty = -ax * h.nz, tz = ax * h.ny - ay * h.nx;  // a x n
+  const float itl = rsqrtf(fmaxf(tx * tx + ty * ty + tz * tz, 1e-20f));
+  tx *= itl;
+  ty *= itl;
+  tz *= itl;
+  return {tx, ty, tz, h.ny * tz - h.nz * ty, h.nz * tx - h.nx * tz, h.nx * ty - h.ny * tx};
+}
+
+// Ambient-occlusion ray a of pixel i.
+__device__ __forceinline__ float ao_ray(const SecParams& k, const SecHit& h, const SecFrame& f, uint32_t i, uint32_t a,
+                                        float* o, float* d) {
+  const uint32_t h0 = hash32(k.seed ^ hash32(i * 0x9E3779B9u + a));
+  const float r1 = unit_float(h0), r2 = unit_float(hash32(h0 ^ 0x68bc21ebu));
+  const float rr = sqrtf(r1), phi = 6.28318530718f * r2;
+  const float lx = rr * cosf(phi), ly = rr * sinf(phi), lz = sqrtf(fmaxf(0.0f, 1.0f - r1));
+  o[0] = h.x + h.nx * k.ao_bias;
+  o[1] = h.y + h.ny * k.ao_bias;
+  o[2] = h.z + h.nz * k.ao_bias;
+  d[0] = lx * f.tx + ly * f.bx + lz * h.nx;
+  d[1] = lx * f.ty + ly * f.by + lz * h.ny;
+  d[2] = lx * f.tz + ly * f.bz + lz * h.nz;
+  return h.hit ? k.ao_radius : -1.0f;
+}
+
 // One thread per ray, in the order of the output arrays: blocks below
 // shadow_blocks write shadow rays, the others ambient-occlusion rays.  Bound by
 // its stores (28 bytes a ray), which a thread per pixel spread over 12-byte
@@ -73,66 +147,13 @@ __global__ void __launch_bounds__(kSecRays) k_secondary(SecParams k) {
   const uint32_t i = static_cast<uint32_t>(i0) + at / per;
   const uint32_t l = at % per;
   const bool live = r0 + threadIdx.x < n;
-  const bool hit = live && (k.flags[i] & RKF_FLAG_HIT) != 0;
+  const SecHit h = load_hit(k, i, live);
   // (the first kind of ray there is counts a pixel)
-  const int hits = __syncthreads_count(hit && l == 0 && (shadow || k.shadow_blocks == 0));
+  const int hits = __syncthreads_count(h.hit && l == 0 && (shadow || k.shadow_blocks == 0));
   if (threadIdx.x == 0 && hits) atomicAdd(k.hits, static_cast<unsigned int>(hits));
-  float hx = 0, hy = 0, hz = 0, nx = 0, ny = 1, nz = 0;
-  if (hit) {
-    const uint32_t px = i % k.w, py = i / k.w;
-    const float u = (static_cast<float>(px) + 0.5f) / static_cast<float>(k.w);
-    const float v = (static_cast<float>(py) + 0.5f) / static_cast<float>(k.h);
-    float dx = k.fwd[0] + (u * 2.0f - 1.0f) * k.right[0] + (1.0f - v * 2.0f) * k.up[0];
-    float dy = k.fwd[1] + (u * 2.0f - 1.0f) * k.right[1] + (1.0f - v * 2.0f) * k.up[1];
-    float dz = k.fwd[2] + (u * 2.0f - 1.0f) * k.right[2] + (1.0f - v * 2.0f) * k.up[2];
-    const float il = rsqrtf(dx * dx + dy * dy + dz * dz);
-    dx *= il;
-    dy *= il;
-    dz *= il;
-    const float t = k.t[i];
-    hx = k.pos[0] + dx * t;
-    hy = k.pos[1] + dy * t;
-    hz = k.pos[2] + dz * t;
-    nx = k.normal[3 * static_cast<size_t>(i)];
-    ny = k.normal[3 * static_cast<size_t>(i) + 1];
-    nz = k.normal[3 * static_cast<size_t>(i) + 2];
-  }
   float* so = sh_o + 3 * threadIdx.x;
   float* sd = sh_d + 3 * threadIdx.x;
-  float tmax;
-  if (shadow) {
-    const float ox = hx + nx * k.shadow_bias, oy = hy + ny * k.shadow_bias, oz = hz + nz * k.shadow_bias;
-    float dx = k.lights[3 * l] - ox, dy = k.lights[3 * l + 1] - oy, dz = k.lights[3 * l + 2] - oz;
-    const float len = sqrtf(dx * dx + dy * dy + dz * dz);
-    const float il = len > 0.0f ? 1.0f / len : 0.0f;
-    so[0] = ox;
-    so[1] = oy;
-    so[2] = oz;
-    sd[0] = dx * il;
-    sd[1] = dy * il;
-    sd[2] = dz * il;
-    tmax = hit ? len : -1.0f;
-  } else {
-    // tangent frame of the normal
-    const float ax = fabsf(nx) < 0.9f ? 1.0f : 0.0f, ay = fabsf(nx) < 0.9f ? 0.0f : 1.0f;
-    float tx = ay * nz, ty = -ax * nz, tz = ax * ny - ay * nx;  // a x n
-    const float itl = rsqrtf(fmaxf(tx * tx + ty * ty + tz * tz, 1e-20f));
-    tx *= itl;
-    ty *= itl;
-    tz *= itl;
-    const float bx = ny * tz - nz * ty, by = nz * tx - nx * tz, bz = nx * ty - ny * tx;
-    const uint32_t h0 = hash32(k.seed ^ hash32(i * 0x9E3779B9u + l));
-    const float r1 = unit_float(h0), r2 = unit_float(hash32(h0 ^ 0x68bc21ebu));
-    const float rr = sqrtf(r1), phi = 6.28318530718f * r2;
-    const float lx = rr * cosf(phi), ly = rr * sinf(phi), lz = sqrtf(fmaxf(0.0f, 1.0f - r1));
-    so[0] = hx + nx * k.ao_bias;
-    so[1] = hy + ny * k.ao_bias;
-    so[2] = hz + nz * k.ao_bias;
-    sd[0] = lx * tx + ly * bx + lz * nx;
-    sd[1] = lx * ty + ly * by + lz * ny;
-    sd[2] = lx * tz + ly * bz + lz * nz;
-    tmax = hit ? k.ao_radius : -1.0f;
-  }
+  const float tmax = shadow ? shadow_ray(k, h, l, so, sd) : ao_ray(k, h, frame_of(h), i, l, so, sd);
   if (live) (shadow ? k.st : k.at)[r0 + threadIdx.x] = tmax;
   __syncthreads();
   const uint32_t words = 3 * static_cast<uint32_t>(n - r0 < kSecRays ? n - r0 : kSecRays);
@@ -141,6 +162,42 @@ __global__ void __launch_bounds__(kSecRays) k_secondary(SecParams k) {
   for (uint32_t e = threadIdx.x; e < words; e += kSecRays) {
     o[e] = sh_o[e];
     d[e] = sh_d[e];
+  }
+}
+
+// A thread per pixel, which takes its point and its tangent frame once: where a
+// pixel has one or two occlusion rays, and at most two shadow rays, its pieces of a
+// line are few enough.  1920x1080, 0+1 / 0+2 / 1+1 / 1+2 / 2+1 / 2+2 lights and occlusion
+// rays: 55 / 76 / 64 / 80 / 85 / 113 us so, 60 / 88 / 76 / 103 / 101 / 126 for a thread per
+// ray; 3+2 225 against 151, 1+4 252 against 163; no occlusion, 1 / 2 / 4 lights 55 / 76 / 250
+// against 51 / 76 / 113.  (A ray's values are stored when all are known: through the
+// functions' pointers 2+1 took 93.)
+constexpr uint32_t kFewRays = 2;
+
+__device__ __forceinline__ void store_ray(float* o, float* d, float* t, size_t r, const float* vo, const float* vd,
+                                          float vt) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) o[3 * r + c] = vo[c];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) d[3 * r + c] = vd[c];
+  t[r] = vt;
+}
+
+__global__ void k_secondary_pixels(SecParams k) {
+  const uint64_t id = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (id >= k.pixels) return;
+  const uint32_t i = static_cast<uint32_t>(id);
+  const SecHit h = load_hit(k, i, true);
+  if (h.hit) atomicAdd(k.hits, 1u);
+  float o[3], d[3];
+  for (uint32_t l = 0; l < k.n_lights; ++l) {
+    const float t = shadow_ray(k, h, l, o, d);
+    store_ray(k.so, k.sd, k.st, static_cast<size_t>(i) * k.n_lights + l, o, d, t);
+  }
+  const SecFrame f = frame_of(h);
+  for (uint32_t a = 0; a < k.ao_per_hit; ++a) {
+    const float t = ao_ray(k, h, f, i, a, o, d);
+    store_ray(k.ao, k.ad, k.at, static_cast<size_t>(i) * k.ao_per_hit + a, o, d, t);
   }
 }
 
@@ -208,7 +265,9 @@ extern "C" rkf_status rkf_secondary_rays(rkf_ctx* ctx, const rkf_camera* cam, ui
   const uint64_t blocks = shadow_blocks + (n * ao_per_hit + detail::kSecRays - 1) / detail::kSecRays;
   if (blocks > 0x7FFFFFFFull) return fail(RKF_INVALID_ARG, "rkf_secondary_rays: too many rays");
   k.shadow_blocks = static_cast<uint32_t>(shadow_blocks);
-  if (blocks) {
+  if (ao_per_hit && ao_per_hit <= detail::kFewRays && n_lights <= detail::kFewRays) {
+    detail::k_secondary_pixels<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(k);
+  } else if (blocks) {
     detail::k_secondary<<<static_cast<unsigned>(blocks), detail::kSecRays, 0, st>>>(k);
   } else {
     detail::k_count_hits<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(k);
