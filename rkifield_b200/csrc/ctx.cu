@@ -213,6 +213,12 @@ rkf_status Ctx::upload_objects() {
   return RKF_OK;
 }
 
+void Ctx::drop_edit_bufs() {
+  spare_top.release();
+  spare_field.release();
+  edit_bufs.clear();
+}
+
 rkf_status Ctx::ensure_leaf_capacity(uint32_t need) {
   if (need <= leaf_cap) return RKF_OK;
   // while serving, in-flight launches hold the leaf buffer's address
@@ -652,8 +658,7 @@ rkf_status rkf_objects_import(rkf_ctx* ctx, const rkf_gpu_object* objects, uint3
   uint32_t cap = 64;
   while (cap < nl) cap *= 2;
   DevBuf nleaves, nleafd, ntop, nfield;
-  c->spare_top.release();  // (of the index this import replaces)
-  c->spare_field.release();
+  c->drop_edit_bufs();
   rkf_status st = nleaves.alloc(static_cast<size_t>(cap) * 2048);
   if (st == RKF_OK) st = nleafd.alloc(static_cast<size_t>(cap) * 512);
   if (st == RKF_OK) st = ntop.alloc(std::max<size_t>(top.size(), 1) * 4);

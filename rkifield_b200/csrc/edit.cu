@@ -536,9 +536,6 @@ extern "C" rkf_status rkf_edit_csg(rkf_ctx* ctx, const rkf_edit_op* op, uint64_t
       c->spare_field.bytes == std::max<uint64_t>(c->top_len, 1)) {
     r.top_dst = c->spare_top.as<uint32_t>();
     r.field_dst = c->spare_field.as<uint8_t>();
-  } else {
-    c->spare_top.release();
-    c->spare_field.release();
   }
   size_t next_buf = 0, kept = 0;
   const EditScratch scratch = [&](size_t bytes) -> void* {
@@ -550,9 +547,11 @@ extern "C" rkf_status rkf_edit_csg(rkf_ctx* ctx, const rkf_edit_op* op, uint64_t
     return b.p;
   };
   rkf_status st = apply_edit(c, *op, c->stream, &r, &scratch);
-  // marches of the old epoch on other streams end before its index is spare,
-  // and error paths may return with work queued
-  RKF_CUDA_TRY(cudaDeviceSynchronize());
+  // Where an epoch was made, marches of the old one on other streams end before
+  // its index is spare and its slots are free.  An edit that failed may have left
+  // work queued; one that was refused or changed nothing waits for nothing.
+  if (st == RKF_OK && r.new_epoch) RKF_CUDA_TRY(cudaDeviceSynchronize());
+  else if (st != RKF_OK && next_buf) RKF_CUDA_TRY(cudaStreamSynchronize(c->stream));
   for (size_t i = 0; i < c->edit_bufs.size(); ++i)
     if ((kept += c->edit_bufs[i]->bytes) > Ctx::kEditKept) {
       c->edit_bufs.resize(i);
@@ -566,7 +565,7 @@ extern "C" rkf_status rkf_edit_csg(rkf_ctx* ctx, const rkf_edit_op* op, uint64_t
     std::swap(c->top.bytes, top.bytes);
     std::swap(c->empty_dist.p, field.p);
     std::swap(c->empty_dist.bytes, field.bytes);
-    if (r.new_top.p) {  // the old epoch's index becomes the spare one
+    if (r.new_top.p) {  // the old epoch's index becomes the spare one (the last spare, of another size, goes)
       std::swap(c->spare_top.p, r.new_top.p);
       std::swap(c->spare_top.bytes, r.new_top.bytes);
       std::swap(c->spare_field.p, r.new_empty_dist.p);
