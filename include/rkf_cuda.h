@@ -331,7 +331,10 @@ typedef struct rkf_bvh_item {
 RKF_API rkf_status rkf_bvh_build(const rkf_bvh_item* items, uint32_t n, rkf_bvh_node* out, uint32_t cap,
                                  uint32_t* n_out);
 
-/* Counts of what the context holds. */
+/* Counts of what the context holds.  device_bytes: the scene, the lists of the
+ * passes before large views (9 bytes a ray, up to 0.6 GB in tiles of 32 rays; outgrown
+ * ones until the index grows or a serving session starts) and the buffers kept between
+ * edits; not what single calls stage. */
 typedef struct rkf_scene_info {
     uint32_t num_objects;
     uint32_t pool_bricks_used;

@@ -213,10 +213,11 @@ rkf_status Ctx::upload_objects() {
   return RKF_OK;
 }
 
-void Ctx::drop_edit_bufs() {
+void Ctx::drop_kept() {
   spare_top.release();
   spare_field.release();
   edit_bufs.clear();
+  settle_old.clear();
 }
 
 rkf_status Ctx::ensure_leaf_capacity(uint32_t need) {
@@ -658,7 +659,7 @@ rkf_status rkf_objects_import(rkf_ctx* ctx, const rkf_gpu_object* objects, uint3
   uint32_t cap = 64;
   while (cap < nl) cap *= 2;
   DevBuf nleaves, nleafd, ntop, nfield;
-  c->drop_edit_bufs();
+  c->drop_kept();
   rkf_status st = nleaves.alloc(static_cast<size_t>(cap) * 2048);
   if (st == RKF_OK) st = nleafd.alloc(static_cast<size_t>(cap) * 512);
   if (st == RKF_OK) st = ntop.alloc(std::max<size_t>(top.size(), 1) * 4);
@@ -760,7 +761,9 @@ rkf_status rkf_scene_info_get(rkf_ctx* ctx, rkf_scene_info* out) {
   out->leaf_blocks = c->n_leaves;
   out->device_bytes = c->dist_f16.bytes + c->dist_f32.bytes + c->dist_u8.bytes + c->brick_step.bytes +
                       c->mat.bytes + c->blend.bytes + c->aos.bytes + c->top.bytes + c->empty_dist.bytes + c->leaves.bytes + c->leaf_dist.bytes +
-                      c->flat_maps.bytes + c->objdev.bytes;
+                      c->flat_maps.bytes + c->objdev.bytes + c->settle_buf.bytes + c->spare_top.bytes + c->spare_field.bytes;
+  for (const auto& b : c->settle_old) out->device_bytes += b->bytes;
+  for (const auto& b : c->edit_bufs) out->device_bytes += b->bytes;
   out->epoch = c->epoch;
   return RKF_OK;
 }

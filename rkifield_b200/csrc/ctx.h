@@ -143,8 +143,9 @@ struct Ctx {
   static constexpr size_t kEditKept = 32u << 20;
   DevBuf spare_top, spare_field;
   std::vector<std::unique_ptr<DevBuf>> edit_bufs;
-  void drop_edit_bufs();  // the index grows, or nothing edits directly for a while: give them back
+  void drop_kept();  // the index grows, or nothing edits directly for a while: give these and settle_old back
   DevBuf settle_buf; // lists of the settling passes (settle.h)
+  std::vector<std::unique_ptr<DevBuf>> settle_old;  // outgrown ones, which a launch under way may use
   DevBuf counters;   // work counters of the persistent kernels
   DevBuf seg_buf;    // segment table of the persistent kernel
 

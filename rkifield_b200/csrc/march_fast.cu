@@ -1757,16 +1757,10 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   // (march timing covers the passes too)
   rkf_status se = c->march_event(st, false);
   if (se != RKF_OK) return se;
-  if (settle && empty && (!tiled_empty || few)) {
-    const size_t need = settle_bytes(view_ids, kp.tile_w * kp.tile_h);
-    if (c->settle_buf.bytes >= need || c->settle_buf.alloc(need + need / 8) == RKF_OK) {
-      const rkf_status s2 = settle_enqueue(c, kp, obj, view_ids, c->settle_buf.p, st);
-      if (s2 != RKF_OK) return s2;
-      if (few) obj = multi_empty ? detail::OBJ_MULTI : detail::OBJ_SINGLE;
-    } else {
-      cudaGetLastError();  // no room for the lists: the march alone
-    }
-  }
+  // (no room for the lists: the march alone)
+  const uint64_t part = settle && empty && (!tiled_empty || few) ? settle_part(c, view_ids, kp.tile_w * kp.tile_h) : 0;
+  const int path = obj;  // the variant the passes settle for
+  if (part && few) obj = multi_empty ? detail::OBJ_MULTI : detail::OBJ_SINGLE;
   if (few && obj == detail::OBJ_SINGLE_EMPTY_TILED) obj = detail::OBJ_SINGLE;
   const void* fn = nullptr;
   switch (c->cfg.precision) {
@@ -1788,13 +1782,26 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
     RKF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
     bps = occ > 0 ? static_cast<uint32_t>(occ) : 1;
   }
-  uint64_t blocks = static_cast<uint64_t>(c->sm_count) * bps;
   const uint64_t block_rays = threads / 32 * detail::kLeastLanes;  // (lane_share spreads them)
-  const uint64_t need_blocks = (total + block_rays - 1) / block_rays;
-  if (blocks > need_blocks) blocks = need_blocks ? need_blocks : 1;
-  void* args[] = {&kp};
-  RKF_CUDA_TRY(cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(threads), args, smem, st));
-  c->counted();
+  for (uint64_t first = 0;;) {
+    // the next part of the views, with the ray batches after the last; or all at once
+    const uint64_t end = part ? std::min(first + part, view_ids) : total;
+    const bool last = !part || end == view_ids;
+    if (part) {
+      if (first) RKF_CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st));
+      const rkf_status s2 = settle_enqueue(c, kp, path, first, end, st);
+      if (s2 != RKF_OK) return s2;
+      kp.total = last ? total : end;
+    }
+    uint64_t blocks = static_cast<uint64_t>(c->sm_count) * bps;
+    const uint64_t need_blocks = ((last ? total : end) - first + block_rays - 1) / block_rays;
+    if (blocks > need_blocks) blocks = need_blocks ? need_blocks : 1;
+    void* args[] = {&kp};
+    RKF_CUDA_TRY(cudaLaunchKernel(fn, dim3(static_cast<unsigned>(blocks)), dim3(threads), args, smem, st));
+    c->counted();
+    if (last) break;
+    first = end;
+  }
   return c->march_event(st, true);
 }
 

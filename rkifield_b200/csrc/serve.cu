@@ -546,7 +546,7 @@ rkf_status rkf_serve_start(rkf_ctx* ctx, const rkf_march_params* p) {
     return fail(RKF_UNSUPPORTED, "rkf_serve_start: serving marches with the brute strategy only");
   RKF_CUDA_TRY(cudaSetDevice(c->device));
   RKF_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  c->drop_edit_bufs();  // (a session's edits have their own)
+  c->drop_kept();  // (a session's edits have their own)
   auto* s = new ServeState();
   s->c = c;
   s->p = *p;

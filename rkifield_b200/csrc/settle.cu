@@ -21,6 +21,8 @@
 // steps, which the walk's bounds decide (else the ray goes to the march).
 #include "settle.h"
 
+#include <algorithm>
+
 #include "empty_dist.h"
 #include "walk.cuh"
 
@@ -32,7 +34,7 @@ struct SettleLists {
   uint32_t* counts;   // [0] tiles listed, [1] rays listed
   uint32_t* tiles;    // tile numbers (view ids / tile area)
   uint2* rays;        // {id, end of the EMPTY samples seen (NaN: none; several objects: no settling before this t)}
-  uint32_t n_tiles;   // of all views
+  uint32_t tile0, n_tiles;  // this part of the views' tiles
 };
 
 // A tile's rays: the centre ray's voxel coordinate g + d t on each axis, and d
@@ -196,9 +198,9 @@ __device__ __forceinline__ Ending tile_ending(const KParams& kp, const Beam& b, 
 // One lane per tile of the launch's views.
 template <bool SINGLE>
 __global__ void __launch_bounds__(128) k_settle_tiles(const __grid_constant__ KParams kp, SettleLists ls) {
-  const uint32_t tile = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
-  const uint32_t area = kp.tile_w * kp.tile_h;
-  const bool live = tile < ls.n_tiles;
+  const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  const uint32_t tile = ls.tile0 + at, area = kp.tile_w * kp.tile_h;
+  const bool live = at < ls.n_tiles;
   const uint32_t seg = live ? find_segment(kp.segs, kp.nseg, static_cast<uint64_t>(tile) * area) : 0u;
   const Segment& sg = kp.segs[seg];
   const uint32_t local = live ? tile - static_cast<uint32_t>(sg.first / area) : 0u;
@@ -368,18 +370,43 @@ __global__ void __launch_bounds__(256) k_settle_rays(const __grid_constant__ KPa
 
 }  // namespace detail
 
-size_t settle_bytes(uint64_t view_ids, uint32_t area) {
-  return 256 + ((view_ids / area * 4 + 255) & ~static_cast<size_t>(255)) + view_ids * 8;
+namespace {
+size_t tile_bytes(uint64_t ids, uint32_t area) { return (ids / area * 4 + 255) & ~static_cast<size_t>(255); }
+}  // namespace
+
+size_t settle_bytes(uint64_t ids, uint32_t area) { return 256 + tile_bytes(ids, area) + ids * 8; }
+
+uint64_t settle_part(Ctx* c, uint64_t view_ids, uint32_t area) {
+  const uint64_t want = std::min(view_ids, kSettlePart / area * area);
+  const size_t need = settle_bytes(want, area);
+  if (c->settle_buf.bytes < need) {
+    // (twice the last size at least, so that views that grow rarely come here; the
+    // last buffer may be in use by a launch under way)
+    const size_t most = settle_bytes(kSettlePart, area);
+    auto grown = std::make_unique<DevBuf>();
+    if (grown->alloc(std::min(std::max(need, 2 * c->settle_buf.bytes), std::max(most, need))) == RKF_OK) {
+      std::swap(grown->p, c->settle_buf.p);
+      std::swap(grown->bytes, c->settle_buf.bytes);
+      if (grown->p) c->settle_old.push_back(std::move(grown));
+    } else {
+      cudaGetLastError();
+    }
+  }
+  if (c->settle_buf.bytes >= need) return want;
+  // (what is left of the buffer: 8 bytes an id, 4 a tile, 512 for the counts and the rounding)
+  const uint64_t tiles = c->settle_buf.bytes > 512 ? (c->settle_buf.bytes - 512) / (8ull * area + 4) : 0;
+  return tiles * area < want / kSettleParts ? 0 : tiles * area;
 }
 
-rkf_status settle_enqueue(Ctx* c, detail::KParams& kp, int obj, uint64_t view_ids, void* ws, cudaStream_t st) {
+rkf_status settle_enqueue(Ctx* c, detail::KParams& kp, int obj, uint64_t first, uint64_t end, cudaStream_t st) {
   const uint32_t area = kp.tile_w * kp.tile_h;
   detail::SettleLists ls;
-  ls.n_tiles = static_cast<uint32_t>(view_ids / area);
-  char* b = static_cast<char*>(ws);
+  ls.tile0 = static_cast<uint32_t>(first / area);
+  ls.n_tiles = static_cast<uint32_t>((end - first) / area);
+  char* b = c->settle_buf.as<char>();
   ls.counts = reinterpret_cast<uint32_t*>(b);
   ls.tiles = reinterpret_cast<uint32_t*>(b + 256);
-  ls.rays = reinterpret_cast<uint2*>(b + 256 + ((view_ids / area * 4 + 255) & ~static_cast<size_t>(255)));
+  ls.rays = reinterpret_cast<uint2*>(b + 256 + tile_bytes(end - first, area));
   RKF_CUDA_TRY(cudaMemsetAsync(ls.counts, 0, 8, st));
   kp.list = nullptr;
   const unsigned blocks = (ls.n_tiles + 127u) / 128u;
@@ -395,7 +422,7 @@ rkf_status settle_enqueue(Ctx* c, detail::KParams& kp, int obj, uint64_t view_id
   RKF_CUDA_TRY(cudaGetLastError());
   kp.list = ls.rays;
   kp.list_n = ls.counts + 1;
-  kp.view_ids = view_ids;
+  kp.view_ids = end;
   return RKF_OK;
 }
 

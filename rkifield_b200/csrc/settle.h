@@ -16,13 +16,23 @@ struct KParams;
 // passes' launches (about 4 us each) cost what they save.
 constexpr uint64_t kSettleIds = 1u << 17;
 
-// Device bytes the passes need for views of view_ids work ids in tiles of
-// `area` of them.
-size_t settle_bytes(uint64_t view_ids, uint32_t area);
+// A launch's views are settled and marched in parts of at most this many ids, which
+// bounds the passes' lists (604 MB in tiles of 32 ids): 32 views of 1920x1080.
+constexpr uint64_t kSettlePart = 1u << 26;
 
-// Enqueues the passes for the launch kp describes (an empty-space variant whose
-// views' ids come first, view_ids of them below 2^32) on st, with their lists
-// in ws, and points kp at what they leave.  obj: the launch's kernel variant.
-rkf_status settle_enqueue(Ctx* c, detail::KParams& kp, int obj, uint64_t view_ids, void* ws, cudaStream_t st);
+// Device bytes the passes need for `ids` work ids in tiles of `area` of them.
+size_t settle_bytes(uint64_t ids, uint32_t area);
+
+// The ids of a part for views of view_ids work ids, a multiple of area or all of
+// them: the context's lists grow for it, or, where there is no room, it is what they
+// hold.  0: no lists, or so small that the views would take more than kSettleParts.
+constexpr uint64_t kSettleParts = 8;
+uint64_t settle_part(Ctx* c, uint64_t view_ids, uint32_t area);
+
+// Enqueues the passes over work ids [first, end) of the launch kp describes (an
+// empty-space variant whose views' ids come first, below 2^32; first a multiple of
+// the tiles' ids) on st, with the context's lists, and points kp at what they leave.
+// obj: the launch's kernel variant.
+rkf_status settle_enqueue(Ctx* c, detail::KParams& kp, int obj, uint64_t first, uint64_t end, cudaStream_t st);
 
 }  // namespace rkf

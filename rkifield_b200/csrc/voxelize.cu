@@ -257,7 +257,7 @@ extern "C" rkf_status rkf_voxelize_prims(rkf_ctx* ctx, const rkf_prim* prims, ui
   Ctx* c = reinterpret_cast<Ctx*>(ctx);
   if (c->obj_count() + 1 > 64) return fail(RKF_UNSUPPORTED, "rkf_voxelize_prims: object table full");
   RKF_CUDA_TRY(cudaSetDevice(c->device));
-  c->drop_edit_bufs();
+  c->drop_kept();
 
   // ---- 1. grid exactly as voxelize_sdf (voxelize_object.rs:61-81) -----------
   VoxGrid g;
