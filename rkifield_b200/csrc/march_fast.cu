@@ -7,18 +7,18 @@
 // (normals), :1036-1112 (ray generation and G-buffer), and
 // shade_common_shading.wgsl:9-33 (soft_shadow).
 //
-// Execution model.  Each lane owns one ray at a time.  A warp alternates
-//   1. refill: idle lanes take the next work ids from a global counter
-//      (one warp-aggregated atomic); ids walk views tile by tile, so a warp's
-//      rays stay spatially coherent;
-//   2. march: up to K sphere-tracing iterations (K = the compaction interval)
-//      in a tight loop, leaving early once no lane is still marching;
-//   3. finish: lanes that hit run their bisection (8 samples) and central
-//      differences (6 samples) together, one sample per iteration;
-//   4. epilogue: finished lanes write their G-buffer entry and go idle.
-// So a ray that ends early frees its lane within K iterations instead of
-// idling it until the slowest ray of the warp finishes.  The hit material is
-// read once, from the position that decided it.
+// Execution model.  Each lane owns one ray at a time and a warp takes one phase at a
+// time, the one most of its lanes are ready for:
+//   refill  once enough lanes are done, they write their outputs and take the next
+//           work ids from a global counter (one warp-aggregated atomic); ids walk
+//           views tile by tile, so a warp's rays stay spatially coherent;
+//   walk    lanes whose last sample was about the EMPTY value find how far their rays
+//           cross EMPTY boxes (walk.cuh), which settles a ray or starts a run;
+//   run     steps over EMPTY samples, without the sampler;
+//   eval    samples of the scene, whatever they are for: a step, a bisection, a
+//           normal's differences.
+// The hit material is read once, from the position that decided it.  Large views come
+// through the passes of settle.cu first, which leave the rays that may hit.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -56,8 +56,7 @@ struct ColdState {
   // multi-object empty-space path: bits 0-7, the voxelized objects of the
   // path (KParams::ev) whose EMPTY runs the ray may take (under the tiled
   // strategy, those its object list holds); bits 8-15, the one whose cube
-  // the ray is in (its last successful probe).  Single-object variants: how
-  // the ray ends if its walk reaches its target (1 past tmax, 2 out of steps).
+  // the ray is in (its last successful probe). 
   // (An odd number of words per lane: a warp's accesses hit 32 distinct banks.)
   uint32_t vox_listed;
 };
@@ -417,7 +416,6 @@ __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, ui
 // 1.64 ms against 1.85 with 5 and 1.73 with 3).
 constexpr uint32_t kRefillLanes = 24;
 constexpr float kShortRun = 8.0f, kPutOff = 8.0f;  // in EMPTY steps
-constexpr uint32_t kWalkLinks = 64;   // boxes a walk takes in one phase
 constexpr uint32_t kLeastLanes = 4;   // lanes a warp fills however few rays there are
 constexpr uint32_t kEvalReps = 8;     // samples a lane takes in one phase
 constexpr int march_blocks(int obj) { return obj >= OBJ_SINGLE_EMPTY_TILED ? 2 : obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
@@ -459,8 +457,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
   ColdState& cs = cold_all[threadIdx.x];
   float ox = 0, oy = 0, oz = 0, rdx = 0, rdy = 0, rdz = 0;
   float t = 0, prev_t = 0, prev_dist = kMaxFloat, tmax = 0;
-  // empty-space path: positions up to here sample the EMPTY value (kNoBox: none;
-  // negative: a walk goes on)
+  // empty-space path: positions up to here sample the EMPTY value (kNoBox: none)
   float box_t = kNoBox;
   float far_t = -1.0f;   // multi-object empty-space path: positions up to here lie outside every ball
   float probe_t = 0.0f;  // empty-space path: no walk before this t
@@ -491,7 +488,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
 
     // ---- the phase most lanes are ready for -----------------------------------
     const bool run = EMPTY_PATH && march && t <= box_t;
-    const bool walk = EMPTY_PATH && march && !run && (box_t < 0.0f || (t >= probe_t && prev_dist >= kp.probe_min));
+    const bool walk = EMPTY_PATH && march && !run && t >= probe_t && prev_dist >= kp.probe_min;
     const bool done = state == ST_IDLE || state == ST_EPI;
     const uint32_t n_done = __popc(__ballot_sync(kFull, done));
     const uint32_t n_walk = EMPTY_PATH ? __popc(__ballot_sync(kFull, walk)) : 0u;
@@ -675,77 +672,44 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
         const float t_hi = (t + k * kp.empty_hi) * (1.0f + grow);
         const bool can = kp.empty_lo >= brk && kp.empty_lo >= near_thr && kp.empty_lo >= min_step;
         if (!MULTI_EMPTY) {
-          // A walk takes kWalkLinks boxes a phase and goes on in the next, so
-          // that lanes that are done make room for new rays meanwhile.  While a
-          // walk goes on, box_t is minus its end, probe_t its target, and the
-          // rest of its state in the cold one.
           const ObjDev& o = sh_objs[0];
           const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
-          float end = -1.0f, out[3];
-          bool more = true;
-          if (box_t < 0.0f) {
-            end = -box_t;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) out[a] = cs.g[a];
-          } else {
-            float t_in, t_out;
-            const bool core = core_interval(o, r, t, t_in, t_out);
-            float target = core ? t_out : -1.0f;
-            if (can) {
-              if (t_lo > tmax) {
-                outcome = 1;
-                target = tmax;
-              } else if (t_hi <= tmax && core && t_out >= t_hi) {
-                outcome = 2;
-                target = t_hi;
-              } else if (OBJ == OBJ_SINGLE_EMPTY) {
-                outcome = leaves_grid(o, r, t, tmax, core, t_out, k, kp.empty_lo_t, kp.empty_hi);
-                if (outcome) target = tmax;
-              }
+          float t_in, t_out;
+          const bool core = core_interval(o, r, t, t_in, t_out);
+          const float run_end = core ? t_out : -1.0f;
+          float target = run_end;
+          uint32_t ends = 0;  // the outcome if the walk reaches its target
+          if (can) {
+            if (t_lo > tmax) {
+              ends = 1;
+              target = tmax;
+            } else if (t_hi <= tmax && core && t_out >= t_hi) {
+              ends = 2;
+              target = t_hi;
+            } else if (OBJ == OBJ_SINGLE_EMPTY) {
+              ends = leaves_grid(o, r, t, tmax, core, t_out, k, kp.empty_lo_t, kp.empty_hi);
+              if (ends) target = tmax;
             }
-            cs.vox_listed = outcome;
-            cs.hi = core ? t_out : -1.0f;  // (the bisection's until then)
-            // outside: nothing to walk for before the ray enters
-            cs.lo = core || (t_in < t_out && t < t_out && !(t_in > t)) ? after(t)
-                    : t_in < t_out && t_in > t ? t_in : after(INFINITY);
-            cs.sub = kp.walk_links;
-            probe_t = target;
-            more = target >= t;
           }
+          // outside: nothing to walk for before the ray enters
+          probe_t = core || (t_in < t_out && t < t_out && !(t_in > t)) ? after(t)
+                    : t_in < t_out && t_in > t ? t_in : after(INFINITY);
           // a tiled step is a coarse skip of more than 0.5 (empty_lo_t is at
           // most that) or evaluates the object: the brute field bounds the
           // ray's samples from below, the tiled one gives their value
-          const bool brute = OBJ == OBJ_SINGLE_EMPTY || cs.vox_listed == 1u;
-          const uint8_t* field = brute ? kp.brute_field : s.empty_dist;
-          if (!(box_t < 0.0f)) {
-            more = more && walk_start(o, s, field, brute, r, t, end, out);
-            if (!more) end = -1.0f;
+          const bool brute = OBJ == OBJ_SINGLE_EMPTY || ends == 1u;
+          float end = -1.0f;
+          if (target >= t) end = walk_empty(o, s, brute ? kp.brute_field : s.empty_dist, brute, r, t, target, kWalkLinks);
+          if (end >= target) outcome = ends;
+          if (OBJ == OBJ_SINGLE_EMPTY_TILED && ends == 1u && !outcome) {
+            // not settled: the tiled field's walk, for a run
+            end = run_end >= t ? walk_empty(o, s, s.empty_dist, false, r, t, run_end, kWalkLinks) : -1.0f;
           }
-          uint32_t links = min(cs.sub, kWalkLinks);
-          cs.sub -= links;
-#pragma unroll 1
-          for (; more && links && end < probe_t; --links) more = walk_link(o, s, field, brute, r, end, out);
-          if (more && end < probe_t && cs.sub) {
-            outcome = 0;
-            box_t = -end;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) cs.g[a] = out[a];
-          } else {
-            outcome = more && end >= probe_t ? cs.vox_listed : 0u;
-            if (OBJ == OBJ_SINGLE_EMPTY_TILED && !outcome && cs.vox_listed == 1u) {
-              // not settled: the tiled field's walk, for a run (this phase
-              // again, with no settling ahead)
-              cs.vox_listed = 3u;
-              end = -1.0f;
-              if (cs.hi >= t) end = walk_empty(o, s, s.empty_dist, false, r, t, cs.hi, kp.walk_links);
-            }
-            box_t = end >= t && cs.hi >= t ? fminf(end, cs.hi) : kNoBox;
-            probe_t = cs.lo;
-            // a walk that brought no run of some length puts the next one off
-            const float from = box_t == box_t ? box_t : t;
-            if (probe_t == probe_t && from - t < kShortRun * kp.empty_hi)
-              probe_t = fmaxf(probe_t, from + kPutOff * kp.empty_hi);
-          }
+          box_t = end >= t && run_end >= t ? fminf(end, run_end) : kNoBox;
+          // a walk that brought no run of some length puts the next one off
+          const float from = box_t == box_t ? box_t : t;
+          if (probe_t == probe_t && from - t < kShortRun * kp.empty_hi)
+            probe_t = fmaxf(probe_t, from + kPutOff * kp.empty_hi);
         } else {
           box_t = kNoBox;
           probe_t = after(t);
@@ -791,7 +755,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
               const bool own = pass || masked;
               if (pass && !(listed && core)) break;
               end = walk_empty(o, s, own ? s.empty_dist : kp.brute_field, !MULTI_TILED || !own, r, t,
-                               pass ? t_out : target, kp.walk_links);
+                               pass ? t_out : target, kWalkLinks);
               if (!pass) {
                 ok = end >= target;
                 exact = exact || (core && t_out >= target);
@@ -1578,7 +1542,6 @@ void empty_bounds(detail::KParams& kp, bool empty, bool multi, bool tiled) {
     kp.empty_hi = e ? std::max(kp.empty_hi, v.empty_hi) : v.empty_hi;
   }
   if (tiled) kp.empty_lo_t = std::min(kp.empty_lo_t, kCoarseNear);
-  kp.walk_links = 64;
 }
 
 constexpr float kFewSteps = 150.0f, kFewStepsTiled = 250.0f;

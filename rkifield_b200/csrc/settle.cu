@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(128) k_settle_tiles(const __grid_constant__ KP
         exact = exact || here.kind != 0u;
         if (!SINGLE && here.kind) end = here;
         const float target = SINGLE || end.kind ? end.target : kp.tiled ? -1.0f : last_step(kp);
-        ok = target >= 0.0f && beam_walk(o, kp.s, kp.brute_field, b, target, kp.walk_links);
+        ok = target >= 0.0f && beam_walk(o, kp.s, kp.brute_field, b, target, kWalkLinks);
       }
       ok = ok && exact && end.kind;
       if (!SINGLE && ok) {
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_settle_rays(const __grid_constant__ KPa
             }
           }
           if (target >= 0.0f) {
-            const float end = walk_empty(o, kp.s, kp.brute_field, true, r, 0.0f, target, kp.walk_links);
+            const float end = walk_empty(o, kp.s, kp.brute_field, true, r, 0.0f, target, kWalkLinks);
             if (!(end >= target)) kind = 0;
             // (the tiled strategy's steps are EMPTY values on its own field only)
             if (!kp.tiled && core && end >= 0.0f) seen = fminf(end, t_out);
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) k_settle_rays(const __grid_constant__ KPa
           for (uint32_t e = 0; ok && e < kp.n_ev; ++e) {
             const ObjDev& o = kp.objs[kp.ev[e].obj];
             const ProbeRay r = probe_ray(o, sg.pos[0], sg.pos[1], sg.pos[2], dx, dy, dz);
-            const float end = walk_empty(o, kp.s, kp.brute_field, true, r, 0.0f, target, kp.walk_links);
+            const float end = walk_empty(o, kp.s, kp.brute_field, true, r, 0.0f, target, kWalkLinks);
             ok = end >= target;
             if (!ok) seen = fmaxf(end, after(0.0f));
             float t_in, t_out;

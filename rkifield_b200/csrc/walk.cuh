@@ -62,6 +62,7 @@ struct FarBall {
 // object of the set samples its EMPTY value and every other object a larger
 // value, so the scene's minimum is the least EMPTY value of the set.
 constexpr uint32_t kMaxEmptyVox = 8;
+constexpr uint32_t kWalkLinks = 64;  // boxes a walk may add
 struct EmptyVox {
   uint32_t obj;       // object index
   uint32_t plain;     // zero translation and unit scale
@@ -91,7 +92,6 @@ struct KParams {
   // objects, and tight bounds of the steps a ray takes over EMPTY samples (a
   // tiled launch's coarse skips, of more than 0.5, included in the lower one)
   float empty_lo, empty_lo_t, empty_hi;
-  uint32_t walk_links;     // empty-space path: boxes a walk may add
   const uint8_t* brute_field;  // empty-space field of the objects alone (s.empty_dist: the tiled launch's)
   const rkf_bvh_node* bvh; // BVH strategy: the imported tree, root first
   const uint32_t* bvh_next;  // per node: the walk's next node (bits 0-30), descend (bit 31)
