@@ -61,6 +61,9 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
                                      const rkf_march_params* p, const rkf_batch_tuning& tu,
                                      cudaStream_t st, Segment* dev_segs, unsigned long long* dev_counter,
                                      bool segs_uploaded = false, bool multi_empty = false);
+// Whether a launch whose views hold view_ids work ids goes through the settling
+// passes (whole launches of launch_persistent on the empty-space path).
+bool launch_settles(const Ctx* c, uint64_t view_ids);
 // Whether a launch over this context's objects with these parameters marches
 // the empty-space path (the condition for ordering its views' tiles), and
 // the object whose empty-space field it reads.

@@ -1562,6 +1562,12 @@ int object_set(const Ctx* c) {
 }
 }  // namespace
 
+bool launch_settles(const Ctx* c, uint64_t view_ids) {
+  const int objs = object_set(c);
+  return (objs == detail::OBJ_SINGLE_EMPTY || objs == detail::OBJ_MULTI_EMPTY) && view_ids >= kSettleIds &&
+         view_ids < (1ull << 32);
+}
+
 bool empty_order_source(const Ctx* c, const rkf_march_params* p, const rkf_batch_tuning& tu, ObjDev* o) {
   if (tu.no_empty_path || p->strategy == RKF_STRATEGY_TILED || c->obj_count() == 0 ||
       c->obj_count() > kMaxObjectsFast)
@@ -1631,8 +1637,7 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   uint64_t view_ids = 0;
   for (const Segment& sg : segs_host)
     if (sg.kind == 0) view_ids += sg.n_ids;
-  const bool settle = (objs == detail::OBJ_SINGLE_EMPTY || objs == detail::OBJ_MULTI_EMPTY) && id0 == 0 &&
-                      !segs_resident && view_ids >= kSettleIds && view_ids < (1ull << 32);
+  const bool settle = !tu.no_empty_path && launch_settles(c, view_ids) && id0 == 0 && !segs_resident;
   if (tu.order_tiles && !settle && id0 == 0 && !segs_resident && !tiled && empty_order_source(c, p, tu, &order_obj)) {
     ordered_segs = segs_host;
     rkf_status s2 = tile_order_prepare(c, ordered_segs, tu.tile_w, tu.tile_h, nullptr, 0, &order_tbl, &ordered);

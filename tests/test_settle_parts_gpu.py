@@ -83,3 +83,17 @@ def test_views_that_settle(ctx, small_scene, size, launches):
     rays = [np.ascontiguousarray(a, np.float32).ravel() for a in _rays(100, seed=1)]
     cam = scenes.seeded_camera(small_scene["spec"], *size, seed=4)
     assert _batch(ctx, cam, *size, rays)[1] == launches
+
+
+def test_autotune_orders_bands_of_settled_views(ctx, small_scene):
+    """The settled launch ignores the tile order, the host bands take it."""
+    from rkifield_b200 import _abi as abi
+    from rkifield_b200 import cudart, engine, scenes
+    w, h = 640, 360
+    keep = cudart.device_gbuffer(w * h)
+    view = (abi.rkf_view * 1)()
+    view[0].camera, view[0].width, view[0].height = scenes.seeded_camera(small_scene["spec"], w, h, seed=4), w, h
+    view[0].out = engine._gb_struct(cudart.gbuffer_ptrs(keep), abi.RKF_MEM_DEVICE)
+    tu = abi.rkf_batch_tuning()
+    abi.check(ctx.lib.rkf_autotune(ctx.h, view, 1, None, 0, C.byref(_params(0)), C.byref(tu)), "autotune")
+    assert tu.order_tiles == 1
