@@ -24,6 +24,12 @@ RKF_API void rkf_testing_fail_allocation_after(long long n);
  * count. */
 RKF_API rkf_status rkf_testing_export_empty_dist(rkf_ctx* ctx, uint8_t* out, uint64_t* n);
 
+/* The same at brick resolution (one byte per leaf entry, indexed like the leaves of
+ * rkf_index_export; defined for leaves the current top grid points at): 0 for a brick
+ * that is not EMPTY, else the Chebyshev distance in bricks to the nearest such brick
+ * of the same object, capped at 8. */
+RKF_API rkf_status rkf_testing_export_leaf_dist(rkf_ctx* ctx, uint8_t* out, uint64_t* n);
+
 /* Number of bands rkf_march uses for a view with host outputs (1 = one
  * launch, then the copies; at most 8), whatever the view's size and whether
  * or not its planes are page-locked; bands < 0 restores the choice by view

@@ -265,6 +265,7 @@ SIGNATURES = {
     "rkf_pool_import_soa": (_I, [_P, _P, _P, _P, _U32, _U32]),
     "rkf_testing_fail_allocation_after": (None, [C.c_longlong]),
     "rkf_testing_export_empty_dist": (_I, [_P, _P, C.POINTER(C.c_uint64)]),
+    "rkf_testing_export_leaf_dist": (_I, [_P, _P, C.POINTER(C.c_uint64)]),
     "rkf_testing_set_host_bands": (None, [C.c_int]),
     "rkf_testing_export_coarse": (_I, [_P, _P, _P, _P, C.POINTER(C.c_uint64)]),
     "rkf_testing_last_variant": (C.c_int, [_P]),

@@ -825,6 +825,16 @@ rkf_status rkf_testing_export_empty_dist(rkf_ctx* ctx, uint8_t* out, uint64_t* n
   return RKF_OK;
 }
 
+rkf_status rkf_testing_export_leaf_dist(rkf_ctx* ctx, uint8_t* out, uint64_t* n) {
+  if (!ctx || !n) return fail(RKF_INVALID_ARG, "rkf_testing_export_leaf_dist: null argument");
+  Ctx* c = reinterpret_cast<Ctx*>(ctx);
+  RKF_CUDA_TRY(cudaSetDevice(c->device));
+  *n = static_cast<uint64_t>(c->n_leaves) * 512;
+  if (out && c->n_leaves)
+    RKF_CUDA_TRY(cudaMemcpy(out, c->leaf_dist.p, static_cast<size_t>(c->n_leaves) * 512, cudaMemcpyDeviceToHost));
+  return RKF_OK;
+}
+
 rkf_status rkf_testing_march_timing(rkf_ctx* ctx, uint32_t enable) {
   if (!ctx || enable > 1) return fail(RKF_INVALID_ARG, "rkf_testing_march_timing: bad argument");
   Ctx* c = reinterpret_cast<Ctx*>(ctx);

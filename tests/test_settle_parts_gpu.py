@@ -85,6 +85,22 @@ def test_views_that_settle(ctx, small_scene, size, launches):
     assert _batch(ctx, cam, *size, rays)[1] == launches
 
 
+def test_tile_order_below_the_passes(ctx, small_scene):
+    """The heaviest-first order where it still acts on a whole launch: three kernels
+    before the march, and the same outputs."""
+    from rkifield_b200 import scenes
+    rays = [np.ascontiguousarray(a, np.float32).ravel() for a in _rays(100, seed=1)]
+    cam = scenes.seeded_camera(small_scene["spec"], 504, 256, seed=6)
+    ref = _general(ctx, cam, 504, 256, rays)
+    tu = ctx.tuning()
+    tu.order_tiles = 1
+    ctx.set_tuning(tu)
+    got, launches = _batch(ctx, cam, 504, 256, rays)
+    assert launches == 4
+    for a, b in zip(got, ref):
+        assert_bits_equal(a, b, "ordered")
+
+
 def test_autotune_orders_bands_of_settled_views(ctx, small_scene):
     """The settled launch ignores the tile order, the host bands take it."""
     from rkifield_b200 import _abi as abi
