@@ -431,15 +431,17 @@ extern "C" rkf_status rkf_voxelize_prims(rkf_ctx* ctx, const rkf_prim* prims, ui
                    kz = static_cast<uint32_t>(blk / (static_cast<size_t>(tdim[0]) * tdim[1]));
     return kx * 8 + 8 <= g.dims[0] && ky * 8 + 8 <= g.dims[1] && kz * 8 + 8 <= g.dims[2];
   };
-  uint32_t n_new_leaves = 0;
+  std::vector<uint32_t> leaf_blocks;  // the object's leaf blocks, in the order of their leaves
   for (size_t blk = 0; blk < ntop; ++blk) {
     if (!n_nonempty[blk]) continue;
     if (n_interior[blk] == 512 && block_full(blk)) {
       top[blk] = RKF_INTERIOR_SLOT;
     } else {
-      top[blk] = c->n_leaves + n_new_leaves++;
+      top[blk] = c->n_leaves + static_cast<uint32_t>(leaf_blocks.size());
+      leaf_blocks.push_back(static_cast<uint32_t>(c->top_len + blk));
     }
   }
+  const uint32_t n_new_leaves = static_cast<uint32_t>(leaf_blocks.size());
   std::vector<uint32_t> leaves(static_cast<size_t>(n_new_leaves) * 512, RKF_EMPTY_SLOT);
   auto put = [&](uint64_t f, uint32_t v) {
     const size_t blk = block_of(f, b3);
@@ -524,10 +526,6 @@ extern "C" rkf_status rkf_voxelize_prims(rkf_ctx* ctx, const rkf_prim* prims, ui
     if (top_off) RKF_CUDA_TRY(cudaMemcpyAsync(nf.p, c->empty_dist.p, top_off, cudaMemcpyDeviceToDevice, c->stream));
     RKF_CUDA_TRY(cudaMemcpyAsync(nt.as<uint32_t>() + top_off, top.data(), ntop * 4, cudaMemcpyHostToDevice, c->stream));
     if ((st = build_empty_dist(od, nt.as<uint32_t>(), nf.as<uint8_t>(), c->stream)) != RKF_OK) return st;
-    std::vector<uint32_t> leaf_blocks;
-    leaf_blocks.reserve(n_new_leaves);
-    for (size_t b = 0; b < ntop; ++b)
-      if (top[b] < RKF_INTERIOR_SLOT) leaf_blocks.push_back(static_cast<uint32_t>(top_off + b));
     if ((st = build_leaf_dist(od, nt.as<uint32_t>(), c->leaves.as<uint32_t>(), c->leaf_dist.as<uint8_t>(),
                               leaf_blocks, c->stream)) != RKF_OK)
       return st;
