@@ -53,7 +53,8 @@ def parse():
     ap.add_argument("--width", type=int, default=1920)
     ap.add_argument("--height", type=int, default=1080)
     ap.add_argument("--cpu-rows", type=int, default=24, help="rows of the view in the CPU sample")
-    ap.add_argument("--sector-rows", type=int, default=16, help="rows used to count algorithmic sectors")
+    ap.add_argument("--sector-rows", type=int, default=16,
+                    help="rows used to count the sectors of a march that steps every sample")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-plain", action="store_true")
     ap.add_argument("--no-sectors", action="store_true")
@@ -1082,10 +1083,14 @@ def run_b200(args, world, rank, local, dist):
             threads = os.cpu_count() or 1
             if not args.no_sectors:
                 st = sector_stats(oracle, sc, cam, p, w, h, sample_rows(h, args.sector_rows), threads)
-                bytes_per_ray = 24.0 + 32.0 * st["sectors"] / st["rays"]
+                # what a launch cannot do without: 24 bytes of outputs a ray.
+                # The sectors a march touches that steps every sample through
+                # the sampler stand beside it: the walks and runs skip most of
+                # them, so they bound nothing here
+                bytes_per_ray = 24.0
                 bytes_launch = bytes_per_ray * n
-                # the march kernel's own launches (the tile-order kernels
-                # before it in each step are not part of its roofline)
+                # the settling passes and the march (tile-order kernels before
+                # a march are not part of it)
                 mean_s = float(np.mean(kernel_ms if kernel_ms else ms)) / 1e3
                 peaks = {}
                 pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -1099,6 +1104,8 @@ def run_b200(args, world, rank, local, dist):
                         "frac": achieved / peak, "traffic": tr,
                         "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)" if peaks else "fallback",
                         "algorithmic_bytes_per_ray": bytes_per_ray,
+                        "traffic_source": "profiles/traffic.json: DRAM bytes of the passes and the march, ncu",
+                        "stepped_bytes_per_ray": 24.0 + 32.0 * st["sectors"] / st["rays"],
                         "sectors_per_ray": st["sectors"] / st["rays"],
                         "index_sectors_per_ray": st["index_sectors"] / st["rays"],
                         "dist_sectors_per_ray": st["dist_sectors"] / st["rays"],

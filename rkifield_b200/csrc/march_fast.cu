@@ -1719,7 +1719,10 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   // 1920x1080, 100 steps: 1.64 ms plain against 2.29; 200 steps: 0.90 either way;
   // 400 steps: 1.15 against 0.59.  Tiled (plain also without the passes):
   // 100 steps 1.30 ms against 5.9, 200 steps 1.08 against 1.47, 400 steps 3.1
-  // against 1.0.
+  // against 1.0.  Views below kSettleIds and ray batches keep the EMPTY variants
+  // (one object, f16, 100 steps; EMPTY / plain us): 160x90 249 / 311, 256x144 372 / 415,
+  // 480x270 544 / 509; 64 / 2,000 / 30,000 / 250,000 rays 88 / 141 / 254 / 694 against 178 /
+  // 239 / 308 / 776.
   const bool few = empty && few_empty_steps(kp, multi_empty, tiled ? kFewStepsTiled : kFewSteps);
   const bool tiled_empty = tiled && empty;
   // (march timing covers the passes too)

@@ -11,9 +11,13 @@ struct KParams;
 
 // A launch's views, when they hold at least this many work ids, go through two
 // passes before the march: one settles whole ray tiles, one the rays of the
-// tiles that are left, and the march takes what remains.  Below it the march
-// alone is as fast: its warps then have no second ray to go on to, so the
-// passes' launches (about 4 us each) cost what they save.
+// tiles that are left, and the march takes what remains.  Below it the march alone
+// is faster: its warps have no second ray to go on to, so what the passes take is
+// added.  us with / without them (default tuning; mean of three cameras), 32 m scene seen
+// from outside: 160x90 413 / 249, 256x144 480 / 372, 400x225 509 / 496, 480x270 557 / 551, 640x360
+// 613 / 599, 960x540 770 / 847, 1280x720 995 / 1,178.  Cameras inside the 1.1M-brick
+// scene, where few tiles settle: 256x144 331 / 268, 480x270 439 / 385, 960x540 643 / 544,
+// 1280x720 717 / 666 -- for such views the line lies too low.
 constexpr uint64_t kSettleIds = 1u << 17;
 
 // A launch's views are settled and marched in parts of at most this many ids, which
