@@ -410,15 +410,17 @@ __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, ui
 //   A walk that brought no run of kShortRun EMPTY steps puts the next one off by
 //   kPutOff: 8 and 8 1,069 / 659 / 3,165 / 426, no putting off 1,157 / 675 /
 //   3,691 / 425, 16 and 16 1,092 / 654 / 3,173 / 432 (with 4 blocks).
-// The variants of several objects and of the tiled strategy hold more state: 2
-// blocks (1277x717, the 1.1M-brick scene and four more objects: 1.42 ms against
-// 1.49 with 4), and their plain kin stay at 4 (u8, 1920x1080 of the 32 m scene:
-// 1.64 ms against 1.85 with 5 and 1.73 with 3).
+// The variants of several objects and of the tiled strategy hold more state, and
+// spill at 4 blocks, but have more samples to wait for (1920x1080 of the 1.1M-brick
+// scene plus 3 voxelized objects and 2 others, brute / tiled / BVH, ms: 4 blocks 6.9 /
+// 7.4 / 7.9, 3 7.8 / 8.0 / 8.3, 2 7.9 / 8.4 / 9.0, 5 7.9 / 7.7 / 8.2; plus 9 others 4.66 / 4.81 /
+// 5.65, 5.10 / 5.02 / 5.57, 5.23 / 4.94 / 6.01, 5.63 / 5.28 / 5.70), as their plain kin (u8,
+// 1920x1080 of the 32 m scene: 1.64 ms with 4 against 1.85 with 5 and 1.73 with 3).
 constexpr uint32_t kRefillLanes = 24;
 constexpr float kShortRun = 8.0f, kPutOff = 8.0f;  // in EMPTY steps
 constexpr uint32_t kLeastLanes = 4;   // lanes a warp fills however few rays there are
 constexpr uint32_t kEvalReps = 8;     // samples a lane takes in one phase
-constexpr int march_blocks(int obj) { return obj >= OBJ_SINGLE_EMPTY_TILED ? 2 : obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
+constexpr int march_blocks(int obj) { return obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
 constexpr uint32_t march_refill(int obj) { return obj == OBJ_MULTI || obj == OBJ_SINGLE ? 16u : kRefillLanes; }
 #define kNoBox __int_as_float(0x7fc00000)  // compares false with every time
 
@@ -728,21 +730,22 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
           }
           // ---- settle: no object below its EMPTY value or ball bound ahead.  Under
           // the tiled strategy running out of steps needs the exact EMPTY value
-          // of an object every step evaluates.
+          // of an object every step evaluates: one the tile lists, on the field of
+          // blocks no coarse skip can reach; what it does not list is not evaluated.
           const bool past = t_lo > tmax;
           const bool masked = MULTI_TILED && !past;
           const float target = past ? tmax : t_hi;
           bool exact = past, ok = can && t >= cs.gpos && far_all >= target &&
-                                  (past || (t_hi <= tmax && (!MULTI_TILED || (cs.vox_listed & 0xFFu) == all)));
+                                  (past || (t_hi <= tmax && (!MULTI_TILED || (cs.vox_listed & 0xFFu) != 0u)));
           const bool tried = ok;
           // ---- run: the set of voxelized objects of the path (that the ray may
           // take runs on) whose EMPTY boxes hold the ray; the run lasts while it
-          // is in all of them
+          // is in all of them, and outside every ball: no walk goes on beyond
           uint32_t set = 0;
           float b = kMaxFloat, walk_at = cs.gpos > t ? cs.gpos : after(INFINITY);  // when to walk again
           for (uint32_t e = 0; e < kp.n_ev && far_all >= 0.0f; ++e) {
             const bool listed = (cs.vox_listed >> e) & 1u;
-            if (!listed && !ok) continue;
+            if (!listed && (!ok || masked)) continue;
             const ObjDev& o = sh_objs[kp.ev[e].obj];
             const ProbeRay r = probe_ray(o, ox, oy, oz, dx, dy, dz);
             float t_in, t_out;
@@ -755,7 +758,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
               const bool own = pass || masked;
               if (pass && !(listed && core)) break;
               end = walk_empty(o, s, own ? s.empty_dist : kp.brute_field, !MULTI_TILED || !own, r, t,
-                               pass ? t_out : target, kWalkLinks);
+                               pass ? fminf(fminf(t_out, b), far_all) : target, kWalkLinks);
               if (!pass) {
                 ok = end >= target;
                 exact = exact || (core && t_out >= target);
