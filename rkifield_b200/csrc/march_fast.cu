@@ -74,20 +74,17 @@ static_assert(sizeof(ColdState) % 8 == 4, "ColdState must span an odd number of 
 // length(clamp(pos, min, max) - pos); its square root is taken only where the
 // comparison needs it (an exact zero stays zero, and any length exceeds a
 // negative best).
-template <int PREC>
-__device__ __forceinline__ float eval_bvh(const SceneDev& s, const ObjDev* objs, const rkf_bvh_node* nodes,
-                                              const uint32_t* __restrict__ next, uint32_t nobj, float wx, float wy,
-                                              float wz, float& best_un, uint32_t& best_i) {
-  LaneCache lc;
-  constexpr uint32_t kEnd = 0x7FFFFFFFu;
-  float best = kMaxFloat;
-  best_un = kMaxFloat;
-  best_i = 0;
-  uint32_t i = 0;
-  while (i != kEnd) {
-    const float4* nd = reinterpret_cast<const float4*>(nodes + i);
+//
+// The next object of that walk for position w and the best value so far; node: where
+// the walk stands (0 at first).  kBvhEnd: none is left.
+constexpr uint32_t kBvhEnd = 0x7FFFFFFFu;
+__device__ __forceinline__ uint32_t bvh_candidate(const rkf_bvh_node* nodes, const uint32_t* __restrict__ next,
+                                                  uint32_t nobj, float wx, float wy, float wz, float best,
+                                                  uint32_t& node) {
+  while (node != kBvhEnd) {
+    const float4* nd = reinterpret_cast<const float4*>(nodes + node);
     const float4 a = __ldg(nd), b = __ldg(nd + 1);
-    const uint32_t link = __ldg(next + i);
+    const uint32_t link = __ldg(next + node);
     const float ex = __fsub_rn(fminf(fmaxf(wx, a.x), b.x), wx);
     const float ey = __fsub_rn(fminf(fmaxf(wy, a.y), b.y), wy);
     const float ez = __fsub_rn(fminf(fmaxf(wz, a.z), b.z), wz);
@@ -96,29 +93,13 @@ __device__ __forceinline__ float eval_bvh(const SceneDev& s, const ObjDev* objs,
     if (d2 == 0.0f) skip = 0.0f > best;
     else if (best < 0.0f && d2 == d2) skip = true;
     else skip = __fsqrt_rn(d2) > best;
-    if (skip) {
-      i = link & kEnd;
-      continue;
-    }
     const uint32_t left = __float_as_uint(a.w), ro = __float_as_uint(b.w);
-    if (left == RKF_BVH_INVALID) {
-      if (ro < nobj) {
-        float du;
-        const float d = eval_obj<PREC>(s, objs[ro], wx, wy, wz, &du, lc);
-        if (d < best) {
-          best = d;
-          best_un = du;
-          best_i = ro;
-        }
-      }
-      i = link & kEnd;
-    } else {
-      i = (link >> 31) ? ro : (link & kEnd);
-    }
+    const bool leaf = left == RKF_BVH_INVALID;
+    node = !skip && !leaf && (link >> 31) ? ro : (link & kBvhEnd);
+    if (!skip && leaf && ro < nobj) return ro;
   }
-  return best;
+  return kBvhEnd;
 }
-
 
 // Up to n march steps of a ray through positions covered by EMPTY boxes: each
 // sample is empty_value().  The run stops before a step whose sample is below
@@ -431,7 +412,7 @@ __device__ __forceinline__ uint32_t lane_share(uint64_t total, uint64_t handed, 
   return max((static_cast<uint32_t>(left) + warps - 1u) / warps, kLeastLanes);
 }
 
-template <int PREC, int OBJ>
+template <int PREC, int OBJ, bool TREE>
 __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(const __grid_constant__ KParams kp) {
   constexpr bool MULTI_TILED = OBJ == OBJ_MULTI_EMPTY_TILED;
   constexpr bool MULTI_EMPTY = OBJ == OBJ_MULTI_EMPTY || MULTI_TILED;
@@ -920,12 +901,16 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
           je = cs.tile_count;
         }
       }
-      if ((!EMPTY_PATH || OBJ == OBJ_MULTI_EMPTY) && kp.use_bvh && state == ST_MARCH) {
-        best = eval_bvh<PREC>(s, sh_objs, kp.bvh, kp.bvh_next, nobj, px, py, pz, best_un, best_i);
-        je = 0;
-      }
-      for (uint32_t j = jb; j < je; ++j) {
-        const uint32_t oi = list ? __ldg(kp.td.tile_list + cs.tile_base + j) : j;
+      const bool tree = TREE && state == ST_MARCH;
+      if (tree) jb = 0u;
+      for (uint32_t j = jb; tree || j < je; ++j) {
+        uint32_t oi = j;
+        if (list) oi = __ldg(kp.td.tile_list + cs.tile_base + j);
+        if (tree) {  // (j: where the walk of the tree stands)
+          oi = bvh_candidate(kp.bvh, kp.bvh_next, nobj, px, py, pz, best, j);
+          if (oi == kBvhEnd) break;
+          --j;
+        }
         const ObjDev& o = sh_objs[SINGLE ? 0u : oi];
         float d = kMaxFloat, du = kMaxFloat;
         if (PLAIN_VOX) {  // one voxelized object, translation only
@@ -1232,16 +1217,21 @@ __global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __r
   }
 }
 
+// The kernel of a launch.  tree: it walks the imported tree (of one object, as of
+// several); the walk's code in the loop of the others cost them 6-10%.
 template <int PREC>
-const void* persistent_fn(int obj) {
-  if (obj == OBJ_MULTI_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY>);
+const void* persistent_fn(int obj, bool tree) {
+  if (tree)
+    return obj == OBJ_MULTI_EMPTY ? reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY, true>)
+                                  : reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI, true>);
+  if (obj == OBJ_MULTI_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY, false>);
   if (obj == OBJ_MULTI_EMPTY_TILED)
-    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY_TILED>);
-  if (obj == OBJ_SINGLE_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY>);
+    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY_TILED, false>);
+  if (obj == OBJ_SINGLE_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY, false>);
   if (obj == OBJ_SINGLE_EMPTY_TILED)
-    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY_TILED>);
-  if (obj == OBJ_SINGLE) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE>);
-  return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI>);
+    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY_TILED, false>);
+  if (obj == OBJ_SINGLE) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE, false>);
+  return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI, false>);
 }
 
 }  // namespace detail
@@ -1702,7 +1692,6 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   kp.tiled = tiled ? 1u : 0u;
   kp.bvh = walk ? c->bvh.as<rkf_bvh_node>() : nullptr;
   kp.bvh_next = walk ? c->bvh_next.as<uint32_t>() : nullptr;
-  kp.use_bvh = walk ? 1u : 0u;
   const ObjDev& e0 = kp.objs[0];  // the object of the single-object empty-space path
   empty_bounds(kp, empty, multi_empty, tiled);
   kp.budget = tu.step_budget ? tu.step_budget : 32;
@@ -1739,13 +1728,13 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
-      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, walk);
       break;
     case RKF_PRECISION_U8:
-      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, walk);
       break;
     default:
-      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, walk);
   }
   c->last_variant = obj;
   kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj);
@@ -1827,13 +1816,13 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
-      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, false);
       break;
     case RKF_PRECISION_U8:
-      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, false);
       break;
     default:
-      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj);
+      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, false);
   }
   c->last_variant = obj;
   const uint32_t threads = tu.threads_per_block ? tu.threads_per_block : 256;  // checked above

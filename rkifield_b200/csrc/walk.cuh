@@ -95,7 +95,6 @@ struct KParams {
   const uint8_t* brute_field;  // empty-space field of the objects alone (s.empty_dist: the tiled launch's)
   const rkf_bvh_node* bvh; // BVH strategy: the imported tree, root first
   const uint32_t* bvh_next;  // per node: the walk's next node (bits 0-30), descend (bit 31)
-  uint32_t use_bvh;
   // multi-object empty-space path: the voxelized objects that take EMPTY
   // runs, and a ball for every object that needs one (bounding the largest
   // EMPTY value of the path)
