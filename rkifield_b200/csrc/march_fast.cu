@@ -400,9 +400,18 @@ __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, ui
 constexpr uint32_t kRefillLanes = 24;
 constexpr float kShortRun = 8.0f, kPutOff = 8.0f;  // in EMPTY steps
 constexpr uint32_t kLeastLanes = 4;   // lanes a warp fills however few rays there are
-constexpr uint32_t kEvalReps = 8;     // samples a lane takes in one phase
 constexpr int march_blocks(int obj) { return obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
-constexpr uint32_t march_refill(int obj) { return obj == OBJ_MULTI || obj == OBJ_SINGLE ? 16u : kRefillLanes; }
+// How a warp is paced: the lanes done before new rays, and the samples a lane takes in
+// one phase (on while half of those that began do).  Without the EMPTY path nearly
+// every lane samples, and a warp does best to stay with it: one rotated object,
+// 1920x1080 of the 32 m scene, f16 / u8, 2.02 / 1.77 ms at 16 lanes and 8 samples, 1.77 / 1.59
+// at 28 and 128; the scene and four more objects, brute / tiled / BVH, 3.30 / 2.57 / 4.88 ms
+// to 3.00 / 2.25 / 4.43 at 28 and 16 to 128.  Of several objects the rays that the settling
+// passes left (listed) go best at 16 lanes: 2.42 ms, at 28 lanes 2.49.
+constexpr uint32_t march_refill(int obj, bool listed) {
+  return obj != OBJ_MULTI && obj != OBJ_SINGLE ? kRefillLanes : obj == OBJ_MULTI && listed ? 16u : 28u;
+}
+constexpr uint32_t eval_reps(int obj) { return obj == OBJ_MULTI ? 16u : obj == OBJ_SINGLE ? 128u : 8u; }
 #define kNoBox __int_as_float(0x7fc00000)  // compares false with every time
 
 // A warp's lanes' share of the ids left to hand out.
@@ -838,7 +847,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
     // ---- eval: a sample of each lane that needs one, and on while most do --------
     bool eval = !done && !walk && !run;
 #pragma unroll 1
-    for (uint32_t rep = 0; rep < kEvalReps; ++rep) {
+    for (uint32_t rep = 0; rep < eval_reps(OBJ); ++rep) {
     if (eval) {
       if (state == ST_BISECT && cs.sub >= p.bisect_steps) {
         // bisection done (or a direct hit): t = (lo+hi)/2, on to the normal
@@ -901,6 +910,8 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
           je = cs.tile_count;
         }
       }
+      // one object's sample counts whatever its value (a NaN, too)
+      const bool take = only || ((SINGLE || (!TREE && nobj == 1u)) && !list);
       const bool tree = TREE && state == ST_MARCH;
       if (tree) jb = 0u;
       for (uint32_t j = jb; tree || j < je; ++j) {
@@ -925,7 +936,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(con
                                                 : sample_vox<PREC>(s, o, lx, ly, lz, grad, lc);
           d = local ? du : __fmul_rn(du, o.min_scale);
         }
-        if ((SINGLE && !list) || only || d < best) {
+        if (take || d < best) {
           best = d;
           best_un = du;
           best_i = oi;
@@ -1725,6 +1736,12 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   const int path = obj;  // the variant the passes settle for
   if (part && few) obj = multi_empty ? detail::OBJ_MULTI : detail::OBJ_SINGLE;
   if (few && obj == detail::OBJ_SINGLE_EMPTY_TILED) obj = detail::OBJ_SINGLE;
+  c->last_variant = obj;
+  const uint32_t refill = detail::march_refill(obj, part != 0);
+  // A view of one object off the EMPTY path, f16 or f32, is faster in the kernel of
+  // several: that of one spills (f16, rotated, 1920x1080 of the 32 m scene 1.68 against
+  // 1.77 ms; u8, which does not, 1.73 against 1.59; 2,000 rays f16 224 against 207 us).
+  if (obj == detail::OBJ_SINGLE && view_ids && c->cfg.precision != RKF_PRECISION_U8) obj = detail::OBJ_MULTI;
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
@@ -1736,8 +1753,7 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
     default:
       fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, walk);
   }
-  c->last_variant = obj;
-  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj);
+  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : refill;
   const size_t smem = 0;
   uint32_t bps = tu.blocks_per_sm;
   if (bps == 0) {
@@ -1810,7 +1826,7 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
   const bool empty = obj == detail::OBJ_SINGLE_EMPTY || memp;
   empty_bounds(kp, empty, memp, false);
   kp.budget = tu.step_budget ? tu.step_budget : 32;
-  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj);
+  kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : detail::march_refill(obj, false);
   kp.brute_field = c->empty_dist.as<uint8_t>();
   kp.plain_obj = (e0.m[12] == 0.0f && e0.m[13] == 0.0f && e0.m[14] == 0.0f && e0.min_scale == 1.0f) ? 1u : 0u;
   const void* fn = nullptr;
