@@ -392,15 +392,20 @@ __device__ __noinline__ void write_unmarched(const Segment& sg, uint32_t idx, ui
 //   kPutOff: 8 and 8 1,069 / 659 / 3,165 / 426, no putting off 1,157 / 675 /
 //   3,691 / 425, 16 and 16 1,092 / 654 / 3,173 / 432 (with 4 blocks).
 // The variants of several objects and of the tiled strategy hold more state, and
-// spill at 4 blocks, but have more samples to wait for (1920x1080 of the 1.1M-brick
+// spill at 4 blocks, but in large views have more samples to wait for (1920x1080 of the 1.1M-brick
 // scene plus 3 voxelized objects and 2 others, brute / tiled / BVH, ms: 4 blocks 6.9 /
 // 7.4 / 7.9, 3 7.8 / 8.0 / 8.3, 2 7.9 / 8.4 / 9.0, 5 7.9 / 7.7 / 8.2; plus 9 others 4.66 / 4.81 /
-// 5.65, 5.10 / 5.02 / 5.57, 5.23 / 4.94 / 6.01, 5.63 / 5.28 / 5.70), as their plain kin (u8,
+// 5.65, 5.10 / 5.02 / 5.57, 5.23 / 4.94 / 6.01, 5.63 / 5.28 / 5.70).  In smaller views the longest
+// rays decide: of the latter 400x225 1.85 / 1.43 / 1.94 with 4, 1.60 / 1.08 / 1.68 with 2, and
+// 960x540 2.53 / 2.25 / 2.63 with 4, 2.39 / 2.16 / 2.62 with 2.  Their plain kin run 4 (u8,
 // 1920x1080 of the 32 m scene: 1.64 ms with 4 against 1.85 with 5 and 1.73 with 3).
 constexpr uint32_t kRefillLanes = 24;
 constexpr float kShortRun = 8.0f, kPutOff = 8.0f;  // in EMPTY steps
 constexpr uint32_t kLeastLanes = 4;   // lanes a warp fills however few rays there are
-constexpr int march_blocks(int obj) { return obj == OBJ_SINGLE_EMPTY ? 3 : 4; }
+constexpr uint64_t kManyIds = 1u << 20;  // work ids of views that count as many
+constexpr int march_blocks(int obj, bool many) {
+  return obj == OBJ_SINGLE_EMPTY ? 3 : obj > OBJ_SINGLE_EMPTY && !many ? 2 : 4;
+}
 // How a warp is paced: the lanes done before new rays, and the samples a lane takes in
 // one phase (on while half of those that began do).  Without the EMPTY path nearly
 // every lane samples, and a warp does best to stay with it: one rotated object,
@@ -421,8 +426,8 @@ __device__ __forceinline__ uint32_t lane_share(uint64_t total, uint64_t handed, 
   return max((static_cast<uint32_t>(left) + warps - 1u) / warps, kLeastLanes);
 }
 
-template <int PREC, int OBJ, bool TREE>
-__global__ void __launch_bounds__(256, march_blocks(OBJ)) k_march_persistent(const __grid_constant__ KParams kp) {
+template <int PREC, int OBJ, bool TREE, bool MANY>
+__global__ void __launch_bounds__(256, march_blocks(OBJ, MANY)) k_march_persistent(const __grid_constant__ KParams kp) {
   constexpr bool MULTI_TILED = OBJ == OBJ_MULTI_EMPTY_TILED;
   constexpr bool MULTI_EMPTY = OBJ == OBJ_MULTI_EMPTY || MULTI_TILED;
   constexpr bool SINGLE = OBJ != OBJ_MULTI && !MULTI_EMPTY;
@@ -1229,20 +1234,23 @@ __global__ void __launch_bounds__(128, 12) k_sdf_ao(SceneDev s, const float* __r
 }
 
 // The kernel of a launch.  tree: it walks the imported tree (of one object, as of
-// several); the walk's code in the loop of the others cost them 6-10%.
-template <int PREC>
+// several); the walk's code in the loop of the others cost them 6-10%.  many: views of
+// kManyIds work ids or more (march_blocks).
+template <int PREC, bool MANY>
 const void* persistent_fn(int obj, bool tree) {
-  if (tree)
-    return obj == OBJ_MULTI_EMPTY ? reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY, true>)
-                                  : reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI, true>);
-  if (obj == OBJ_MULTI_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY, false>);
-  if (obj == OBJ_MULTI_EMPTY_TILED)
-    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI_EMPTY_TILED, false>);
-  if (obj == OBJ_SINGLE_EMPTY) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY, false>);
-  if (obj == OBJ_SINGLE_EMPTY_TILED)
-    return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE_EMPTY_TILED, false>);
-  if (obj == OBJ_SINGLE) return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_SINGLE, false>);
-  return reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ_MULTI, false>);
+#define RKF_MARCH(OBJ, TREE, MANY) reinterpret_cast<const void*>(&k_march_persistent<PREC, OBJ, TREE, MANY>)
+  if (obj == OBJ_MULTI_EMPTY) return tree ? RKF_MARCH(OBJ_MULTI_EMPTY, true, MANY) : RKF_MARCH(OBJ_MULTI_EMPTY, false, MANY);
+  if (tree) return RKF_MARCH(OBJ_MULTI, true, false);
+  if (obj == OBJ_MULTI_EMPTY_TILED) return RKF_MARCH(OBJ_MULTI_EMPTY_TILED, false, MANY);
+  if (obj == OBJ_SINGLE_EMPTY_TILED) return RKF_MARCH(OBJ_SINGLE_EMPTY_TILED, false, MANY);
+  if (obj == OBJ_SINGLE_EMPTY) return RKF_MARCH(OBJ_SINGLE_EMPTY, false, false);
+  if (obj == OBJ_SINGLE) return RKF_MARCH(OBJ_SINGLE, false, false);
+  return RKF_MARCH(OBJ_MULTI, false, false);
+#undef RKF_MARCH
+}
+template <int PREC>
+const void* persistent_fn(int obj, bool tree, bool many) {
+  return many ? persistent_fn<PREC, true>(obj, tree) : persistent_fn<PREC, false>(obj, tree);
 }
 
 }  // namespace detail
@@ -1738,6 +1746,7 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   if (few && obj == detail::OBJ_SINGLE_EMPTY_TILED) obj = detail::OBJ_SINGLE;
   c->last_variant = obj;
   const uint32_t refill = detail::march_refill(obj, part != 0);
+  const bool many = view_ids >= detail::kManyIds;
   // A view of one object off the EMPTY path, f16 or f32, is faster in the kernel of
   // several: that of one spills (f16, rotated, 1920x1080 of the 32 m scene 1.68 against
   // 1.77 ms; u8, which does not, 1.73 against 1.59; 2,000 rays f16 224 against 207 us).
@@ -1745,13 +1754,13 @@ rkf_status launch_persistent(Ctx* c, const std::vector<Segment>& segs_host, uint
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
-      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, walk);
+      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, walk, many);
       break;
     case RKF_PRECISION_U8:
-      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, walk);
+      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, walk, many);
       break;
     default:
-      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, walk);
+      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, walk, many);
   }
   kp.refill_idle = tu.refill_idle && tu.refill_idle < 32u ? tu.refill_idle : refill;
   const size_t smem = 0;
@@ -1832,13 +1841,13 @@ rkf_status launch_persistent_scratch(Ctx* c, const Segment* segs_host, uint32_t 
   const void* fn = nullptr;
   switch (c->cfg.precision) {
     case RKF_PRECISION_F32:
-      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, false);
+      fn = detail::persistent_fn<RKF_PRECISION_F32>(obj, false, false);
       break;
     case RKF_PRECISION_U8:
-      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, false);
+      fn = detail::persistent_fn<RKF_PRECISION_U8>(obj, false, false);
       break;
     default:
-      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, false);
+      fn = detail::persistent_fn<RKF_PRECISION_F16>(obj, false, false);
   }
   c->last_variant = obj;
   const uint32_t threads = tu.threads_per_block ? tu.threads_per_block : 256;  // checked above
