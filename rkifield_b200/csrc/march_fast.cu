@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(256, march_blocks(OBJ, MANY)) k_march_persiste
         // several objects: the set's EMPTY values (of one object, its constants)
         const uint32_t set = MULTI_EMPTY ? (cs.vox_listed >> 8) : 1u;
         const bool one = (set & (set - 1u)) == 0u;
-        const EmptyVox& ev = kp.ev[MULTI_EMPTY ? (__ffs(set | 1u) - 1) : 0];
+        const EmptyVox& ev = kp.ev[MULTI_EMPTY && set ? (__ffs(set) - 1) : 0];  // (the one of a set of one)
         const ObjDev& o0 = sh_objs[MULTI_EMPTY ? ev.obj : 0u];
         const uint32_t plain = MULTI_EMPTY ? (one ? ev.plain : 0u) : kp.plain_obj;
         // (the path's least lower bound: no set's is below it)
