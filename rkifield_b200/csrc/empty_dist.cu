@@ -71,7 +71,7 @@ __global__ void k_empty_dist_lower(uint8_t* __restrict__ field, GridDims g, cons
   const uint32_t x = lo.x + static_cast<uint32_t>(i % ext.x);
   const uint32_t y = lo.y + static_cast<uint32_t>((i / ext.x) % ext.y);
   const uint32_t z = lo.z + static_cast<uint32_t>(i / (static_cast<uint64_t>(ext.x) * ext.y));
-  const uint64_t cell = x + static_cast<uint64_t>(y) * g.nx + static_cast<uint64_t>(z) * g.nx * g.ny;
+  const uint64_t cell = g.off + x + static_cast<uint64_t>(y) * g.nx + static_cast<uint64_t>(z) * g.nx * g.ny;
   uint32_t v = field[cell];
   for (uint32_t b = 0; b < nb && v > 0; ++b) {
     const uint32_t l = blocks[b] - g.off;

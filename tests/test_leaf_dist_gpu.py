@@ -61,3 +61,30 @@ def test_distances_and_interior_edits(small_scene):
             for eye, to in ((at, at + np.array([1.0, 0.3, 0.2])), (np.array([14.0, 3.0, 9.0]), at)):
                 got = _both(ctx, scenes.camera_uniforms(eye, to, w, h), _params(0), w, h)
                 assert ((got["flags"] & 1) != 0).any()
+
+
+def test_block_field_of_a_second_object(small_scene):
+    """An edit lowers the block distances of its own object, wherever its grid lies
+    in the field: exact around additive edits in each of two objects, and the views of
+    both are those of the general path."""
+    from rkifield_b200 import scenes
+    from rkifield_b200.engine import Context
+    from test_empty_dist_gpu import _chebyshev, _field
+    from test_multi_vox_gpu import _moved
+    with Context(pool_capacity=200_000, keep_reference_pool=False) as ctx:
+        for k in range(2):
+            prims = small_scene["prims"][5 * k:5 * k + 5].copy()
+            ctx.voxelize(prims, scenes.voxelize_params(small_scene["spec"], prims, object_id=k + 1))
+        ctx.update_objects([ctx.object(0), _moved(ctx.object(1), (40.0, 3.0, -2.0), 2)], [0, 1])
+        rng = np.random.default_rng(5)
+        for k in (1, 0, 1):
+            half = 0.4 * np.array([ctx.object(k).brick_map_dims[a] for a in range(3)]) * 0.32
+            at = rng.uniform(-half, half)
+            op = _op(0, at, 0.7, 3)
+            op.object_index = k
+            ctx.edit(op)
+            idx = ctx.export_index()
+            field, want = _field(ctx), _chebyshev(idx["top"], idx["obj_top_info"])
+            assert (field <= want).all() and ((field == 0) == (want == 0)).all()
+            to = at + (np.array([40.0, 3.0, -2.0]) if k else 0.0)
+            _both(ctx, scenes.camera_uniforms(to + np.array([6.0, 4.0, 7.0]), to, 521, 256), _params(0), 521, 256)
