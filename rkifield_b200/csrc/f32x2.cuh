@@ -2,7 +2,9 @@
 // instructions (PTX add/sub/mul/fma .rn.f32x2, PTX ISA 8.6).  Each lane of a
 // pair is rounded exactly as the scalar instruction rounds it (IEEE
 // round-to-nearest-even, no flush of subnormals), so a packed chain gives the
-// same bits as the scalar chain it replaces, in half the instructions.
+// same bits as the scalar chain it replaces, in half the instructions --
+// except that the assembler may join f2_mul and an f2_add or f2_sub of its result into
+// one fma (seen with CUDA 12.9, .rn notwithstanding): take such a product by scalars.
 #pragma once
 
 #include <cstdint>

@@ -160,7 +160,11 @@ __device__ __forceinline__ uint32_t empty_run(const ObjDev& o, float ox, float o
 // operations on the same values, so the same bits.
 __device__ __forceinline__ float empty_value_x2(f2 o01, f2 d01, f2 h01, f2 r2, f2 nvs2, f2 half2, float oz, float dz,
                                                 float hz, float vs, float rcp, float be, float t) {
-  const f2 g01 = f2_add(f2_add(o01, f2_mul(d01, f2_pack(t, t))), h01);
+  // (the products one at a time: the assembler joins a packed product and the packed
+  // sum that takes it into one instruction, which rounds once)
+  float dx, dy;
+  f2_unpack(d01, dx, dy);
+  const f2 g01 = f2_add(f2_add(o01, f2_pack(__fmul_rn(dx, t), __fmul_rn(dy, t))), h01);
   const f2 q0 = f2_mul(g01, r2);
   const f2 v01 = f2_sub(f2_fma(f2_fma(q0, nvs2, g01), r2, q0), half2);
   const float vz = __fsub_rn(exact_div_vs(__fadd_rn(__fadd_rn(oz, __fmul_rn(dz, t)), hz), vs, rcp), 0.5f);
